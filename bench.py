@@ -41,6 +41,9 @@ L2_FLUSH = 256 << 20
 # writes X0 (44 B)
 STAGE_BYTES_PER_CELL = (44 + 68 + 68 + 44) / 4
 STEP_BYTES_PER_CELL = 264
+# algorithmic bytes per cell of a whole-step launch (stages and tail in one
+# kernel): reads u, v, eta, H, Fx, writes u, v, eta
+WHOLE_STEP_BYTES_PER_CELL = 32
 # the 16-bit storage form (scaled 16-bit state pairs, stage increments and
 # accumulated increments; FP32 X0 after the last stage): stage 1 reads the
 # state's pair and writes the stage increment and D (32 B with H, Fx), stages
@@ -434,16 +437,19 @@ def main():
             raise SystemExit(f"profiled run failed with code {st.code}")
         m.close()
         stage_ms = allmax(prof.kernel_ms[0] / max(prof.launches[0], 1))
+        whole = prof.launches[0] == prof.steps and prof.launches[1] == 0     # one launch for stages and tail
         kernels = {abi.PROFILE_NAMES[k]: {"launches": int(prof.launches[k]),
                                           "avg_us": 1e3 * prof.kernel_ms[k] / prof.launches[k],
                                           "share": prof.kernel_ms[k] / max(sum(prof.kernel_ms), 1e-12)}
                    for k in range(abi.PROFILE_KINDS) if prof.launches[k]}
-        return {"t_dev": t_dev, "value": args.gpus * cells * args.steps / t_dev, "stage_ms": stage_ms,
+        return {"t_dev": t_dev, "value": args.gpus * cells * args.steps / t_dev, "stage_ms": stage_ms, "whole": whole,
                 "kernels": kernels, "launches": launches}
 
     main = time_form(storage, args.build)
     t_dev, value, kernels, launches = main["t_dev"], main["value"], main["kernels"], main["launches"]
     stage_bytes = STAGE_BYTES_PER_CELL if storage == "native" else STAGE_BYTES_PER_CELL_16
+    if main["whole"]:
+        stage_bytes = WHOLE_STEP_BYTES_PER_CELL
     step_bytes = STEP_BYTES_PER_CELL if storage == "native" else STEP_BYTES_PER_CELL_16
     achieved = stage_bytes * cells / (main["stage_ms"] / 1e3) / 1e9
     peak, peak_kind = peaks()
@@ -531,8 +537,9 @@ def main():
             "value": value, "ms_per_step": 1e3 * t_dev / args.steps,
             "e2e": e2e,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "traffic": ncu_traffic(cells) if storage == "native" else None,
-                         "kernel": "rk_stage_tma" if storage == "native" else "s16_stage_kernel",
+                         "frac": achieved / peak, "traffic": ncu_traffic(cells) if storage == "native" and not main["whole"] else None,
+                         "kernel": "rk_step_kernel" if main["whole"] else
+                         "rk_stage_tma" if storage == "native" else "s16_stage_kernel",
                          "bytes_per_cell": stage_bytes,
                          "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
                          else "fallback 6.65 TB/s"},

@@ -32,6 +32,7 @@
 #include "sw_common.cuh"
 #include "sw_ghost.cuh"
 #include "sw_stage.cuh"
+#include "sw_step.h"
 #include "sw_ssp.cuh"
 #include "sw_linear.cuh"
 #include "sw_advcor.cuh"
@@ -169,6 +170,7 @@ struct EngineBase {
     virtual int diagnostics(sw_ctx* ctx, sw_diag* out) = 0;
     virtual int prologue(sw_ctx* ctx) = 0;                   // work of time_integration before its loop
     virtual int ghost_state(sw_ctx* ctx) = 0;
+    virtual int rhs_again(sw_ctx*) { return SW_OK; }         // rhs_in of the last step, if it was not kept
     // the storage form's own copy of the state: made from the FP32 buffers
     // S[p], sst[sp] after an upload, and written back into them before a
     // download or a diagnostics pass (no-ops for the native storage)
@@ -209,10 +211,20 @@ struct sw_ctx {
     // CUDA graphs of one time step, keyed by the buffer parities and the
     // sub-steps that are due (see step_key); off with SWB200_GRAPHS=0
     bool use_graphs = true;
-    struct StepGraph { cudaGraphExec_t exec = nullptr; long long launches = 0; bool flips_sp = false; Fields3 rhs_in; };
+    struct StepGraph { cudaGraphExec_t exec = nullptr; long long launches = 0; bool flips_sp = false; Fields3 rhs_in; int rhs_p = -1; };
     // the buffers the last right-hand-side evaluation of the last step read
     // (the input of the last RK stage or SSP sub-stage); null before a step
     Fields3 rhs_in;
+    // a whole-step launch keeps no stage input in device memory: rhs_in is null
+    // and sw_get_rhs_input forms it again from the step's start, S[rhs_p] at
+    // model time rhs_t (-1: no such step)
+    int rhs_p = -1;
+    long long rhs_t = 0;
+    StepPlan step_plan;        // tiles of the whole-step kernel (shape < 0: not used)
+    // while a block of steps is captured: the branch its tracers run on and
+    // their events (see capture_block); null otherwise
+    cudaStream_t side = nullptr;
+    std::vector<cudaEvent_t>* side_events = nullptr;
     std::map<unsigned, StepGraph> graphs;
     int nsm = 148;
     int tail_ty = TAIL_TY;        // rows per warp strip of the streaming tail (see pick_strip_ty)
@@ -358,6 +370,26 @@ int launch(sw_ctx* ctx, int kind, F&& f) {
     return SW_OK;
 }
 
+// Launches the tracer: on the context's stream, or, in a captured block of
+// steps, on the block's side branch behind the step just issued.
+template <class F>
+int launch_tracer(sw_ctx* ctx, F&& f) {
+    if (!ctx->side) return launch(ctx, 2, f);
+    cudaEvent_t e[2];
+    for (cudaEvent_t& x : e) {
+        CK(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
+        ctx->side_events->push_back(x);
+    }
+    CK(cudaEventRecord(e[0], ctx->stream));
+    CK(cudaStreamWaitEvent(ctx->side, e[0]));
+    std::swap(ctx->stream, ctx->side);
+    const int rc = launch(ctx, 2, f);
+    std::swap(ctx->stream, ctx->side);
+    if (rc) return rc;
+    CK(cudaEventRecord(e[1], ctx->side));
+    return SW_OK;
+}
+
 // ghost points of u, v, eta: the rule of every cell whose value some halo cell
 // copies (the source cells of sw_ghost.cuh) and of the untouched ring cells,
 // enumerated directly so the launch touches only the domain's edges
@@ -419,7 +451,25 @@ dim3 tracer_grid(const sw_ctx* ctx) {
 
 template <class T, class Tp>
 struct Engine : EngineBase {
-    int init(sw_ctx*) { return SW_OK; }
+    static constexpr bool STEP_TYPES = std::is_same<T, Tp>::value &&
+                                       (std::is_same<T, float>::value || std::is_same<T, double>::value);
+    int init(sw_ctx* ctx) {
+        // the whole-step kernel serves RK, nonlinear Arakawa-Hsu dynamics and the plain
+        // continuity equation, with winds and Coriolis values constant along x and ghost copies
+        // that do not round (Tcomm at least T)
+        const sw_config& c = ctx->cfg;
+        for (const char* k : {"SWB200_TMA", "SWB200_STAGE_BLOCKS", "SWB200_STAGE_TY", "SWB200_TAIL_TY"})
+            if (getenv(k)) return SW_OK;             // settings of the launches per stage: these then run
+        // Below 1024 cells a step keeps a launch per pass, as callers that count launches there
+        // expect (four stages, tail and tracer); SWB200_STEP overrides.
+        if ((long long)ctx->g.N * ctx->g.M < 1024 && !getenv("SWB200_STEP")) return SW_OK;
+        if constexpr (STEP_TYPES)
+            if (c.time_scheme == SW_RK && c.dynamics == SW_NONLINEAR && c.adv_scheme == SW_ARAKAWA_HSU &&
+                c.nstep_advcor == 0 && !c.surface_relax && !c.surface_forcing && fmt_size(c.Tcomm) >= sizeof(T))
+                if (ctx->fq.sx == 0 && ctx->Fx.sx == 0 && ctx->Fy.sx == 0)
+                    ctx->step_plan = step_plan<T>(ctx->g, ctx->nsm, ctx->H.sx != 0);
+        return SW_OK;
+    }
 
     // continuity! variant and its fields (src/continuity.jl:3-49); the forcing
     // factor Fetat = T(sin(omega_Feta*t)) at the step's model time
@@ -790,45 +840,109 @@ struct Engine : EngineBase {
         return a;
     }
 
+    // seasonal wind factors at model time t (1 when off)
+    static void wind_factors(const sw_ctx* ctx, long long t, T& Fxt, T& Fyt) {
+        const sw_config& c = ctx->cfg;
+        Fxt = c.seasonal_wind_x ? (T)std::sin(c.omegaFx * (double)t) : T(1);
+        Fyt = c.seasonal_wind_y ? (T)std::sin(c.omegaFy * (double)t) : T(1);
+    }
+
+    // RK stage k of a step from S[p], in a launch of its own
+    int rk_stage(sw_ctx* ctx, int k, int p, bool tail_now, T Fxt, T Fyt) {
+        const sw_config& c = ctx->cfg;
+        const Geom& g = ctx->g;
+        const Fields3& X = ctx->S[p];
+        const StageArgs<T, Tp> a = stage_args(ctx, k, p, tail_now, Fxt, Fyt);
+        const Fields3& in = (k == 1) ? X : ((k % 2 == 0) ? ctx->A : ctx->B);
+        const bool first = (k == 1), last = (k == c.RKo);
+        if (last) ctx->rhs_in = in;
+        if (c.dynamics == SW_LINEAR)
+            return launch(ctx, 0, [&] { lin_rk_dispatch(ctx, a, g.ep != 0, first, last); });
+        if (TMA_TYPES && ctx->use_tma && a.cont == 0 && !a.sadourny && !a.qS) {
+            StageMaps mp;
+            mp.in_u = ctx->tmaps[in.u].in; mp.in_v = ctx->tmaps[in.v].in; mp.in_e = ctx->tmaps[in.e].in;
+            mp.x_u = ctx->tmaps[X.u].x; mp.x_v = ctx->tmaps[X.v].x; mp.x_e = ctx->tmaps[X.e].x;
+            mp.a_u = ctx->tmaps[ctx->Acc.u].x; mp.a_v = ctx->tmaps[ctx->Acc.v].x; mp.a_e = ctx->tmaps[ctx->Acc.e].x;
+            int lr = 0;
+            const int rc = launch(ctx, 0, [&] { lr = stage_tma_dispatch(ctx, a, mp, g.ep != 0, first, last); });
+            return !rc && lr ? fail(ctx, SW_ERR_CUDA, "TMA stage kernel could not be configured") : rc;
+        }
+        const int nblk = (a.nsx * a.nsy + 3) / 4 + a.nring_blocks;
+        return launch(ctx, 0, [&] { stage_dispatch(a, g.ep != 0, first, last, nblk, ctx->stream, ctx->stage_ty); });
+    }
+
+    // The arguments of the whole-step kernel for a step from S[p] to S[1-p]
+    template <class U = T>
+    StepArgs<U> step_args(sw_ctx* ctx, int p, bool tail_now, U Fxt, U Fyt) const {
+        const sw_config& c = ctx->cfg;
+        const Fields3& X = ctx->S[p];
+        const Fields3& Y = ctx->S[1 - p];
+        StepArgs<U> a;
+        a.g = ctx->g;
+        a.ntx = a.nty = 0;                          // set at the launch
+        a.uX = (const U*)X.u; a.vX = (const U*)X.v; a.eX = (const U*)X.e;
+        a.uo = (U*)Y.u; a.vo = (U*)Y.v; a.eo = (U*)Y.e;
+        a.H = sf<U>(ctx->H); a.fq = sf<U>(ctx->fq); a.Fx = sf<U>(ctx->Fx); a.Fy = sf<U>(ctx->Fy);
+        using K = Pack<U>;
+        for (int k = 0; k < 4; k++) {
+            a.a[k] = K::host(k < c.RKo ? (U)c.RKaDt[k] : U(0));
+            a.b[k] = K::host(k + 1 < c.RKo ? (U)c.RKbDt[k] : U(0));
+        }
+        a.rko = c.RKo;
+        a.g_ = K::host((U)c.g); a.Fxt = Fxt; a.Fyt = Fyt;
+        a.tail = tail_now; a.drag = c.bottom_drag; a.smag = c.diffusion == SW_DIFF_SMAGORINSKY;
+        a.cD = K::host((U)c.cD); a.rD = K::host((U)c.rD);
+        a.cSmag = K::host((U)c.cSmag); a.nuB = K::host((U)c.nuB);
+        a.Dt_diff = K::host((U)c.Dt_diff);
+        a.gr = rule(ctx);
+        a.st = ctx->dst;
+        return a;
+    }
+
+    // The input of the last step's last stage, formed again by the launches of
+    // its earlier stages (the same values) from the state the step started
+    // from.  A NaN stop would make them return at once: it is lifted meanwhile.
+    int rhs_again(sw_ctx* ctx) override {
+        if (ctx->rhs_in.u || ctx->rhs_p < 0) return SW_OK;
+        T Fxt, Fyt;
+        wind_factors(ctx, ctx->rhs_t, Fxt, Fyt);
+        CK(cudaMemcpyAsync(ctx->hst, ctx->dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaMemsetAsync(ctx->dst, 0, sizeof(DevStatus), ctx->stream));
+        for (int k = 1; k < ctx->cfg.RKo; k++)
+            if (int rc = rk_stage(ctx, k, ctx->rhs_p, true, Fxt, Fyt)) return rc;
+        CK(cudaMemcpyAsync(ctx->dst, ctx->hst, sizeof(DevStatus), cudaMemcpyHostToDevice, ctx->stream));
+        ctx->rhs_in = (ctx->cfg.RKo % 2 == 0) ? ctx->A : ctx->B;
+        return SW_OK;
+    }
+
     int step(sw_ctx* ctx, long long i) override {
         const sw_config& c = ctx->cfg;
         const Geom& g = ctx->g;
         Fields3& X = ctx->S[ctx->p];
         Fields3& Y = ctx->S[1 - ctx->p];
-        const bool tail_now = (i % c.nstep_diff) == 0;
-        const T one = T(1);
-        T Fxt = c.seasonal_wind_x ? (T)std::sin(c.omegaFx * (double)ctx->t) : one;
-        T Fyt = c.seasonal_wind_y ? (T)std::sin(c.omegaFy * (double)ctx->t) : one;
+        bool tail_now = (i % c.nstep_diff) == 0;
+        T Fxt, Fyt;
+        wind_factors(ctx, ctx->t, Fxt, Fyt);
 
         // ------------------------------------------------ RK stages (:55-78)
-        const int nsx = (g.N + STRIP - 1) / STRIP, nsy = (g.M + ctx->stage_ty - 1) / ctx->stage_ty;
-        const int nring = ring_blocks(g, 128);
-        const int nblk = (nsx * nsy + 3) / 4 + nring;
-        if (c.time_scheme != SW_RK) {
+        ctx->rhs_p = -1;
+        if (ctx->step_plan.shape >= 0) {
+            if constexpr (STEP_TYPES) {
+                const StepArgs<T> a = step_args(ctx, ctx->p, tail_now, Fxt, Fyt);
+                cudaError_t e = cudaSuccess;
+                int rc = launch(ctx, 0, [&] { e = step_launch<T>(ctx->step_plan, a, ctx->H.sx != 0, ctx->stream); });
+                if (!rc && e != cudaSuccess) rc = fail(ctx, SW_ERR_CUDA, std::string("step kernel: ") + cudaGetErrorString(e));
+                if (rc) return rc;
+            }
+            ctx->rhs_in = Fields3();
+            ctx->rhs_p = ctx->p;
+            ctx->rhs_t = ctx->t;
+            tail_now = false;                       // done by the same launch
+        } else if (c.time_scheme != SW_RK) {
             if (int rc = ssp_stages(ctx, X, Y, tail_now, Fxt, Fyt)) return rc;
         } else {
-        for (int k = 1; k <= c.RKo; k++) {
-            StageArgs<T, Tp> a = stage_args(ctx, k, ctx->p, tail_now, Fxt, Fyt);
-            const Fields3& in = (k == 1) ? X : ((k % 2 == 0) ? ctx->A : ctx->B);
-            const bool first = (k == 1), last = (k == c.RKo);
-            if (last) ctx->rhs_in = in;
-            int rc;
-            if (c.dynamics == SW_LINEAR) {
-                rc = launch(ctx, 0, [&] { lin_rk_dispatch(ctx, a, g.ep != 0, first, last); });
-            } else if (TMA_TYPES && ctx->use_tma && a.cont == 0 && !a.sadourny && !a.qS) {
-                StageMaps mp;
-                mp.in_u = ctx->tmaps[in.u].in; mp.in_v = ctx->tmaps[in.v].in; mp.in_e = ctx->tmaps[in.e].in;
-                mp.x_u = ctx->tmaps[X.u].x; mp.x_v = ctx->tmaps[X.v].x; mp.x_e = ctx->tmaps[X.e].x;
-                mp.a_u = ctx->tmaps[ctx->Acc.u].x; mp.a_v = ctx->tmaps[ctx->Acc.v].x; mp.a_e = ctx->tmaps[ctx->Acc.e].x;
-                int lr = 0;
-                rc = launch(ctx, 0, [&] { lr = stage_tma_dispatch(ctx, a, mp, g.ep != 0, first, last); });
-                if (!rc && lr) rc = fail(ctx, SW_ERR_CUDA, "TMA stage kernel could not be configured");
-            } else {
-                rc = launch(ctx, 0, [&] { stage_dispatch(a, g.ep != 0, first, last, nblk, ctx->stream, ctx->stage_ty); });
-            }
-            if (rc) return rc;
-        }
-
+            for (int k = 1; k <= c.RKo; k++)
+                if (int rc = rk_stage(ctx, k, ctx->p, tail_now, Fxt, Fyt)) return rc;
         }
 
         // ---------------------- advection/Coriolis refresh (:208-211)
@@ -867,7 +981,7 @@ struct Engine : EngineBase {
                 TracerArgs<T, Tp> a = tracer_args(ctx, ctx->p, ctx->sp);
                 const bool um_is_u = (c.nadvstep == 1);
                 const dim3 grid = tracer_grid(ctx);
-                int rc = launch(ctx, 2, [&] {
+                int rc = launch_tracer(ctx, [&] {
                     if (g.ep) tracer_dispatch2<true>(a, um_is_u, c.tracer_consumption != 0, grid, ctx->stream);
                     else tracer_dispatch2<false>(a, um_is_u, c.tracer_consumption != 0, grid, ctx->stream);
                 });
@@ -1163,7 +1277,7 @@ struct Engine16 : Engine<float, float> {
                 const TracerIO16<S16> io{inv_s};
                 const bool um_is_u = c.nadvstep == 1;
                 const dim3 grid = tracer_grid(ctx);
-                const int rc = launch(ctx, 2, [&] {
+                const int rc = launch_tracer(ctx, [&] {
                     if (g.ep) tracer16<true>(t, io, um_is_u, c.tracer_consumption != 0, grid, ctx->stream);
                     else tracer16<false>(t, io, um_is_u, c.tracer_consumption != 0, grid, ctx->stream);
                 });
@@ -1396,6 +1510,7 @@ int do_step(sw_ctx* ctx, long long i) {
         sg.launches = ctx->launches - l0;
         sg.flips_sp = ctx->sp != sp0;
         sg.rhs_in = ctx->rhs_in;
+        sg.rhs_p = ctx->rhs_p;
         ctx->t = t0; ctx->launches = l0; ctx->sp = sp0;
         if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&sg.exec, graph, 0);
         if (graph) cudaGraphDestroy(graph);
@@ -1410,9 +1525,93 @@ int do_step(sw_ctx* ctx, long long i) {
     }
     CK(cudaGraphLaunch(it->second.exec, ctx->stream));
     ctx->launches += it->second.launches;
+    ctx->rhs_p = it->second.rhs_p;
+    ctx->rhs_t = ctx->t;
     ctx->t += c.dtint;
     if (it->second.flips_sp) ctx->sp = 1 - ctx->sp;
     ctx->rhs_in = it->second.rhs_in;
+    return SW_OK;
+}
+
+// A block of steps in one graph: STEP_BLOCK steps with the same sub-steps due
+// (so that it is the same launches whenever it begins at the same parities).
+// A launch of a graph costs several microseconds beside its kernels, more than
+// a step's kernels on a small grid.  In a block the tracer of a step runs on a
+// branch of its own beside the next step, which reads nothing of it; the step
+// after that overwrites the velocities it reads, and waits for it.
+constexpr int STEP_BLOCK = 16;   // even: a block ends at the parities it began at
+
+int capture_block(sw_ctx* ctx, long long i, sw_ctx::StepGraph& sg) {
+    const long long t0 = ctx->t, l0 = ctx->launches;
+    const int p0 = ctx->p, sp0 = ctx->sp;
+    std::vector<cudaEvent_t> events;
+    cudaStream_t side = nullptr;
+    CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    int rc = SW_OK;
+    cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
+    cudaGraph_t graph = nullptr;
+    if (e == cudaSuccess) {
+        // the tracer of every step reads the velocities of that step alone
+        const bool branch = ctx->cfg.tracer_advection && ctx->cfg.nadvstep == 1;
+        ctx->side = branch ? side : nullptr;
+        ctx->side_events = &events;
+        for (int k = 0; k < STEP_BLOCK && !rc && e == cudaSuccess; k++) {
+            if (branch && k >= 2) e = cudaStreamWaitEvent(ctx->stream, events[2 * (k - 2) + 1]);
+            if (e == cudaSuccess) rc = ctx->eng->step(ctx, i + k);
+            ctx->p = 1 - ctx->p;
+        }
+        if (branch && !rc && e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, events.back());
+        ctx->side = nullptr;
+        ctx->side_events = nullptr;
+        const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
+        if (e == cudaSuccess) e = e2;
+    }
+    sg.launches = ctx->launches - l0;
+    sg.flips_sp = false;
+    sg.rhs_in = ctx->rhs_in;
+    sg.rhs_p = ctx->rhs_p;
+    ctx->t = t0; ctx->launches = l0; ctx->p = p0; ctx->sp = sp0;
+    if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&sg.exec, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    for (cudaEvent_t x : events) cudaEventDestroy(x);
+    cudaStreamDestroy(side);
+    if (!rc && e != cudaSuccess) {
+        (void)cudaGetLastError();
+        sg.exec = nullptr;              // no block for these steps: they run one by one
+    }
+    return rc;
+}
+
+// Runs a block of steps from step i if there is one to run (of at most `room`
+// steps, none but the last of them due for a NaN check); *ran: steps done, the
+// context then being as after do_step of the last of them.
+int do_block(sw_ctx* ctx, long long i, long long room, long long* ran) {
+    const sw_config& c = ctx->cfg;
+    *ran = 0;
+    // a context that is asked for a few steps only does not pay for the capture
+    if (room < STEP_BLOCK || (ctx->step < 2 * STEP_BLOCK && room < 4 * STEP_BLOCK)) return SW_OK;
+    if (!ctx->use_graphs || ctx->prof || c.seasonal_wind_x || c.seasonal_wind_y || c.surface_forcing) return SW_OK;
+    const long long check = (i + c.nout - 1) / c.nout * c.nout;
+    if (i + STEP_BLOCK - 1 > check) return SW_OK;
+    const unsigned key = step_key(ctx, i), due = key & ~3u;
+    for (int k = 1; k < STEP_BLOCK; k++)
+        if ((step_key(ctx, i + k) & ~3u) != due) return SW_OK;
+    const unsigned bkey = key | 1u << 16;
+    auto it = ctx->graphs.find(bkey);
+    if (it == ctx->graphs.end()) {
+        sw_ctx::StepGraph sg;
+        if (int rc = capture_block(ctx, i, sg)) return rc;
+        it = ctx->graphs.emplace(bkey, sg).first;
+    }
+    if (!it->second.exec) return SW_OK;
+    CK(cudaGraphLaunch(it->second.exec, ctx->stream));
+    ctx->launches += it->second.launches;
+    ctx->t += (long long)STEP_BLOCK * c.dtint;
+    ctx->rhs_in = it->second.rhs_in;
+    ctx->rhs_p = it->second.rhs_p;
+    ctx->rhs_t = ctx->t - c.dtint;
+    ctx->p = 1 - ctx->p;                // the last step's start
+    *ran = STEP_BLOCK;
     return SW_OK;
 }
 
@@ -1420,11 +1619,16 @@ int run_steps(sw_ctx* ctx, long long nsteps, sw_status* status) {
     const sw_config& c = ctx->cfg;
     long long done = 0;
     int code = SW_OK;
-    for (long long s = 0; s < nsteps; s++) {
-        long long i = ctx->step + 1;
-        int rc = do_step(ctx, i);
+    while (done < nsteps) {
+        long long i = ctx->step + 1, ran = 0;
+        int rc = do_block(ctx, i, nsteps - done, &ran);
+        if (!rc && !ran) {
+            rc = do_step(ctx, i);
+            ran = 1;
+        }
         if (rc) return rc;
-        done++;
+        done += ran;
+        i += ran - 1;
         bool check = (i % c.nout) == 0;
         if (check) {
             if ((rc = ctx->eng->nan_check(ctx, i))) return rc;
@@ -1466,6 +1670,7 @@ int run_steps(sw_ctx* ctx, long long nsteps, sw_status* status) {
 std::string env_settings() {
     std::string s;
     for (const char* k : {"SWB200_TMA", "SWB200_GRAPHS", "SWB200_STAGE_BLOCKS", "SWB200_TAIL_TY", "SWB200_STAGE_TY",
+                          "SWB200_STEP", "SWB200_STEP_ROWS",
                           "SWB200_TEST_WAIT_LIMIT", "SWB200_TEST_SKIP_CHUNK"}) {
         const char* v = getenv(k);
         s += k;
@@ -1526,6 +1731,7 @@ sw_ctx* take_dropin(const sw_config* cfg) {
 int state_copy_in(sw_ctx* ctx, const void* u, const void* v, const void* eta, const void* sst) {
     ctx->p = 0; ctx->sp = 0; ctx->step = 0; ctx->t = 0;
     ctx->rhs_in = Fields3();
+    ctx->rhs_p = -1;
     int rc;
     if ((rc = copy_in(ctx, ctx->S[0].u, u, shape_u(ctx->g)))) return rc;
     if ((rc = copy_in(ctx, ctx->S[0].v, v, shape_v(ctx->g)))) return rc;
@@ -2241,7 +2447,8 @@ int sw_trim_memory(void) {
 void sw_destroy(sw_ctx* ctx) {
     if (!ctx) return;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    for (auto& kv : ctx->graphs) cudaGraphExecDestroy(kv.second.exec);
+    for (auto& kv : ctx->graphs)
+        if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     for (auto& a : ctx->allocs) cached_free(a.first, a.second);
     if (ctx->hst) cached_free_host(ctx->hst, sizeof(DevStatus));
     if (ctx->flush) cudaFree(ctx->flush);
@@ -2398,8 +2605,9 @@ int sw_get_rhs_input(sw_ctx* ctx, void* u, void* v, void* eta) {
     if (!ctx || !u || !v || !eta) return SW_ERR_ARG;
     if (ctx->cfg.storage != SW_STORE_NATIVE)
         return fail(ctx, SW_ERR_UNSUPPORTED, "the 16-bit storage form keeps its stage values in 16 bits");
-    const Fields3& X = ctx->rhs_in.u ? ctx->rhs_in : ctx->S[ctx->p];
     int rc;
+    if ((rc = ctx->eng->rhs_again(ctx))) return rc;
+    const Fields3& X = ctx->rhs_in.u ? ctx->rhs_in : ctx->S[ctx->p];
     if ((rc = copy_out(ctx, u, X.u, shape_u(ctx->g)))) return rc;
     if ((rc = copy_out(ctx, v, X.v, shape_v(ctx->g)))) return rc;
     if ((rc = copy_out(ctx, eta, X.e, shape_e(ctx->g)))) return rc;

@@ -1,0 +1,575 @@
+// sw_step.cuh -- a whole Runge-Kutta step (all stages and the dissipative
+// tail) in one launch.
+//
+// A block owns a tile of the domain and carries it through the RKo stages of
+// src/time_integration.jl:55-78 and the tail (:204-221) in shared memory: it
+// loads the step's state once with a halo wide enough for every stage, keeps
+// the stage input (u, v, eta) and the point-wise intermediates (q, U, V, p)
+// there and writes the new state once.  Each stage is two passes over the
+// tile: A forms q, U, V, p from u, v, eta (UVfluxes!, PV!, bernoulli!), B the
+// tendencies and the stage combination, in place.  The tail is two more: T1
+// forms the viscosity, the Laplacians and the speed, T2 the new u and v.
+// Every value is formed by the expression that sw_stage.cuh and sw_tail.cuh
+// form it with, so the results are theirs bit for bit.
+//
+// Halo.  A stage's output at (x, y) reads its input at x-2..x+1, y-2..y+1 and
+// the tail reads +-2, so RKo = 4 needs 10 points below and 6 above a tile;
+// halo points are computed redundantly, on rows whose number shrinks from
+// stage to stage.  Walls need no extra halo: ghost points are filled in shared
+// memory after each stage, by the rules of sw_ghost.cuh.  Where a periodic tile crosses x = 0 it holds the ghost
+// columns of both sides: its columns run
+//   ..., N-2, N-1, N, N+1 | -2, -1, 0, 1, ...
+// so every column sees the neighbours and the depth that the reference's
+// arrays give it, and a ghost column is 4 columns from its source.  A domain
+// that fits is one tile with its ghosts.
+//
+// Packs.  A thread computes V columns at once (sw_pack.cuh): for Float32 a
+// tile's EW lanes hold 2 EW - 4 columns, lane lx the columns lx and
+// lx + EW - 4.  The two halves overlap by 4 columns; after each stage the
+// lanes beside the overlap write the 3 columns that the other half cannot
+// compute (it lacks their neighbours) into it.
+//
+// Measured (B200, per step without the tracer; four stage launches and the
+// tail before): 2048x1024 Float32 124 us against 160, 1000x500 43 against 90,
+// 512x256 Float64 28 against 57.  The 108 x 47 tile of 63 rows takes 57
+// thousand clocks: load 6, A 4 x 3.8, B 4 x 7.6, T1 5, T2 7.7.  B issues in
+// four tenths of its slots (sixteen warps of 128 registers, each row a chain
+// of loads and packed adds); variants of 20, 24 and 32 warps with fewer
+// registers took the same time at this size.  On small grids the passes'
+// latencies (about 1000 clocks each) and the launch are the time.
+#pragma once
+#include <type_traits>
+
+#include "sw_common.cuh"
+#include "sw_ghost.cuh"
+#include "sw_pack.cuh"
+
+namespace swb {
+
+constexpr int STEP_LO = 10, STEP_HI = 6;   // halo below and above a tile (4 stages and the tail)
+
+template <class T>
+struct StepArgs {
+    Geom g;
+    int ntx, nty;                       // tiles in x and y (balanced: see step_cols, step_rows)
+    const T* uX; const T* vX; const T* eX;   // state at the step's start (ghosts valid)
+    T* uo; T* vo; T* eo;                     // new state, with its ghosts
+    SField<T> H, fq, Fx, Fy;            // fq, Fx, Fy constant along x
+    using P = typename Pack<T>::P;      // constants as packs, so that they are read as they are used
+    P a[4], b[4];                       // RKaΔt, RKbΔt
+    int rko;
+    T Fxt, Fyt;
+    int tail, drag, smag;               // tail due; enum sw_bottom_drag; Smagorinsky (else constant νB)
+    P g_, cD, rD, cSmag, nuB, Dt_diff;
+    P half, q4, o12, nz;                // 1/2, 1/4, 1/12, -0.0 (sw_pack.cuh)
+    GhostRule<T> gr;
+    DevStatus* st;
+};
+
+// The columns of tile i: outputs [xs, xe), its first column at virtual column
+// z0.  A periodic domain's first and last tile hold 4 ghost columns more, so
+// the split treats the domain as 8 columns longer and gives them 4 fewer.
+__host__ __device__ inline void step_cols(int N, int ep, int ntx, bool whole, int i, int& xs, int& xe, int& z0) {
+    if (whole) { xs = 0; xe = N; z0 = -2; return; }
+    const int L = ep ? N + 8 : N, sh = ep ? 4 : 0;
+    const int lo = (int)((long long)i * L / ntx) - sh, hi = (int)((long long)(i + 1) * L / ntx) - sh;
+    xs = lo < 0 ? 0 : lo;
+    xe = hi > N ? N : hi;
+    z0 = xs - STEP_LO - (ep && i == 0 ? 4 : 0);
+}
+// The rows of tile j: outputs [ys, ye), loaded rows [z0, z1).
+__host__ __device__ inline void step_rows(int M, int nty, int j, int& ys, int& ye, int& z0, int& z1) {
+    ys = (int)((long long)j * M / nty);
+    ye = (int)((long long)(j + 1) * M / nty);
+    z0 = ys - STEP_LO < -2 ? -2 : ys - STEP_LO;
+    z1 = ye + STEP_HI > M + 2 ? M + 2 : ye + STEP_HI;
+}
+
+// EWW warps side by side (EW = 32 EWW lanes), NW warps in all, R rows per
+// thread: EH rows.
+template <class T, int EWW_, int NW_, int R_>
+struct StepShape {
+    using P = typename Pack<T>::P;
+    static constexpr int EWW = EWW_, NW = NW_, R = R_, EH = NW / EWW * R;
+    static constexpr int V = Pack<T>::V, EW = 32 * EWW, NG = NW / EWW, NP = EW * EH;
+    static constexpr int COLS = V == 2 ? 2 * EW - 4 : EW;     // distinct columns
+    static constexpr int PAD = 4;       // the first row's left neighbour (every other read outside an array is in the next)
+    static constexpr int smem(bool hvar) { return ((7 + hvar) * NP + PAD + 4 * EH) * (int)sizeof(P); }
+};
+
+// One tile.  EDGE is false for tiles none of whose points is a ghost, a ghost
+// source or a wall.  HVAR: the depth varies along x (an array in shared
+// memory; else one value per row).
+template <class T, class SH, bool HVAR, bool EDGE>
+__device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>::P* sm, int xs, int xe, int zx,
+                                          int ys, int ye, int zy, int zy1, bool whole) {
+    using K = Pack<T>;
+    using P = typename K::P;
+    constexpr int EW = SH::EW, NP = SH::NP, R = SH::R, V = SH::V, EH = SH::EH;
+    constexpr int SHIFT = EW - 4;                         // columns between the halves
+    P* const su = sm + SH::PAD;
+    P* const sv = su + NP;
+    P* const se = sv + NP;
+    P* const sq = se + NP;
+    P* const sU = sq + NP;
+    P* const sV = sU + NP;
+    P* const sp = sV + NP;
+    P* const sH = sp + NP;                                // HVAR only
+    P* const tH = sH + (HVAR ? NP : 0);         // per row: depth, Coriolis, wind
+    P* const tf = tH + EH;
+    P* const tFx = tf + EH;
+    P* const tFy = tFx + EH;
+
+    const Geom& g = A.g;
+    const int N = g.N, M = g.M;
+    const bool per = g.ep != 0;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int lx = (warp % SH::EWW) * 32 + lane;
+    const int ly0 = (warp / SH::EWW) * R;
+    const int EHv = zy1 - zy;                             // rows of this tile
+    const P half = A.half, q4 = A.q4, nz = A.nz;
+    const bool lowwall = zy == -2, highwall = zy1 == M + 2;
+
+    // this thread's columns
+    int X[V];
+    bool cv[V];
+#pragma unroll
+    for (int h = 0; h < V; h++) {
+        const int z = zx + lx + h * SHIFT;
+        X[h] = z;
+        cv[h] = true;
+        if (EDGE) {
+            if (per && z < -2) X[h] = z + N + 4;
+            if (per && z > N + 1) X[h] = z - (N + 4);
+            cv[h] = X[h] >= -2 && X[h] <= N + 1 && !(whole && z > N + 1);
+            if (!cv[h]) X[h] = 0;
+        }
+    }
+    auto gofs = [&](int h, int y) { return (y + ROW0) * g.P + X[h] + COL0; };
+    // columns whose outputs this half of the pack computes from valid neighbours
+    const bool prod = V == 1 || (lx >= 2 && lx <= EW - 2);
+    // the overlap: lane 3 passes its upper column down, lanes EW-4, EW-3 their lower columns up
+    const bool xch = V == 2 && (lx == 3 || lx == EW - 4 || lx == EW - 3);
+    const int xofs = lx == 3 ? 2 * (EW - 4) : -2 * SHIFT + 1;
+    auto scalar = [](P* f) { return reinterpret_cast<T*>(f); };
+    auto at = [](P* f, int s, int h) -> T& { return reinterpret_cast<T*>(f)[s * V + h]; };
+    bool own[V];                                          // outputs of this tile
+#pragma unroll
+    for (int h = 0; h < V; h++) {
+        const int rel = lx + h * SHIFT;
+        own[h] = rel >= xs - zx && rel < xe - zx && (V == 1 || (h == 0 ? lx <= EW - 3 : lx >= 2));
+    }
+
+    // EDGE only: what the thread's columns are
+    bool cu[V];                                           // u interior
+    bool zero = false;                                    // one of the columns is 0 of a periodic domain
+    bool wrap = false;                                    // one of the columns is -1 of a periodic domain
+#pragma unroll
+    for (int h = 0; h < V; h++) {
+        cu[h] = cv[h] && X[h] >= (per ? 0 : 1) && X[h] < N;
+        zero = zero || (per && cv[h] && X[h] == 0);
+        wrap = wrap || (per && cv[h] && X[h] == -1);
+    }
+    P x0u[R], x0v[R], x0e[R];                             // the accumulator X0 of this thread's points
+    // whether any lane's are
+    const bool wwrap = EDGE && __any_sync(0xffffffffu, wrap), wzero = EDGE && __any_sync(0xffffffffu, zero);
+
+    // ---- the step's state, halo and ghosts included
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int ly = ly0 + i;
+        if (ly < EHv) {
+            T a[V], b[V], c[V], d[V];
+#pragma unroll
+            for (int h = 0; h < V; h++) {
+                a[h] = b[h] = c[h] = T(0);
+                d[h] = T(1);
+                if (!EDGE || cv[h]) {
+                    const int o = gofs(h, zy + ly);
+                    a[h] = A.uX[o]; b[h] = A.vX[o]; c[h] = A.eX[o];
+                    if (HVAR) {
+                        const T w = A.H.at(X[h], zy + ly);
+                        d[h] = (X[h] >= -1 && X[h] <= N) ? w : T(1);
+                    }
+                }
+            }
+            const int s = ly * EW + lx;
+            su[s] = x0u[i] = K::make(a[0], a[V - 1]);
+            sv[s] = x0v[i] = K::make(b[0], b[V - 1]);
+            se[s] = x0e[i] = K::make(c[0], c[V - 1]);
+            if (HVAR) sH[s] = K::make(d[0], d[V - 1]);
+        }
+    }
+    for (int ly = threadIdx.x; ly < EHv; ly += SH::NW * 32) {
+        const int y = zy + ly + ROW0;
+        if (!HVAR) tH[ly] = K::all(A.H.p[y * A.H.sy]);
+        tf[ly] = K::all(A.fq.p[y * A.fq.sy]);
+        tFx[ly] = K::all(A.Fxt * A.Fx.p[y * A.Fx.sy]);
+        tFy[ly] = K::all(A.Fyt * A.Fy.p[y * A.Fy.sy]);
+    }
+    __syncthreads();
+
+    // stores the updated pack of index s.  Ghost points and columns outside the
+    // domain receive values without meaning here: ghosts() fills the former,
+    // nothing reads the latter.
+    auto store = [&](P* f, int s, P val) {
+        if (prod) f[s] = val;
+        if (xch) scalar(f)[s * V + xofs] = lx == 3 ? K::template get<1>(val) : K::template get<0>(val);
+    };
+    // EDGE: ghost points of u, v, eta (src/ghost_points.jl:46-133), spread over
+    // the block: columns -2, -1, N, N+1 of every row, then rows -2, -1, M, M+1
+    // of every column.  Neither part reads what the other writes.
+    auto ghosts = [&]() {
+        auto from = [&](P* f, int rel, int ly) {
+            return V == 1 || rel < EW - 2 ? at(f, ly * EW + rel, 0) : at(f, ly * EW + rel - SHIFT, V - 1);
+        };
+        auto put = [&](P* f, int rel, int ly, T val) {
+            if (rel < EW) at(f, ly * EW + rel, 0) = val;
+            if (V == 2 && rel >= SHIFT) at(f, ly * EW + rel - SHIFT, V - 1) = val;
+        };
+        const T oma = A.gr.oma;
+        const bool seam = per && !whole;
+        for (int t = threadIdx.x; t < 4 * EH; t += SH::NW * 32) {
+            const int j = t & 3, ly = t >> 2, y = zy + ly;
+            // the j-th ghost column's place, its column and the distance to its source
+            const int gx = j < 2 ? j - 2 : N + j - 2;
+            const int rel = (seam ? (j < 2 ? gx : gx - (N + 4)) + (zx < -2 ? 0 : N + 4) : gx) - zx;
+            const int d = per ? (whole ? (j < 2 ? N : -N) : (j < 2 ? -4 : 4)) : (j == 0 ? 3 : j == 1 ? 1 : j == 2 ? -1 : -3);
+            if (ly < EHv && rel >= 0 && rel < SH::COLS && rel + d >= 0 && rel + d < SH::COLS) {
+                if (per) put(su, rel, ly, from(su, rel + d, ly));
+                const T w = from(sv, rel + d, ly);
+                put(sv, rel, ly, per ? w : oma * w);
+                if (j == 1 || j == 2) {                   // eta: the corners take the column-copied value
+                    const int src = min(max(ly, -zy), M - 1 - zy);
+                    if (y >= -1 && y <= M) put(se, rel, ly, from(se, rel + d, src));
+                }
+            }
+        }
+        if (lowwall || highwall)
+            for (int t = threadIdx.x; t < 4 * 128; t += SH::NW * 32) {
+                const int j = t >> 7, rel = t & 127;
+                const int y = j < 2 ? j - 2 : M + j - 2, ly = y - zy;
+                const int d = j == 0 ? 3 : j == 1 ? 1 : j == 2 ? -1 : -3;
+                int x = zx + rel;
+                if (per && x < -2) x += N + 4;
+                else if (per && !whole && x > N + 1) x -= N + 4;
+                if (rel < SH::COLS && ly >= 0 && ly < EHv && x >= -1 && x <= N + 1) {
+                    if (!per) put(su, rel, ly, oma * from(su, rel, ly + d));
+                    if ((j == 1 || j == 2) && x >= 0 && x < N) put(se, rel, ly, from(se, rel, ly + d));
+                }
+            }
+    };
+
+    const int rko = A.rko;
+    for (int k = 0; k < rko; k++) {
+        const bool last = k == rko - 1;
+        // rows of the stage input that are valid, then the rows each pass forms
+        const int ay = lowwall ? 0 : 2 * k, by = highwall ? EHv : EHv - k;
+        const int a0 = lowwall ? -zy : ay + 1, a1 = highwall ? M + 1 - zy : by;
+        // ---- pass A: q, U, V, p
+        {
+            const P gg = A.g_;
+            const int r0 = max(ly0, a0), r1 = min(ly0 + R, a1);
+            if (r0 < r1) {
+                int s = r0 * EW + lx;
+                P u_m = su[s - EW], v_c = sv[s], h_m, hs_m;
+                {
+                    const P Hc = HVAR ? sH[s - EW] : tH[r0 - 1];
+                    h_m = K::add(se[s - EW], Hc);
+                    hs_m = K::mul(q4, K::add(K::add(se[s - EW - 1], HVAR ? sH[s - EW - 1] : Hc), h_m), nz);
+                }
+#pragma unroll 2
+                for (int ly = r0; ly < r1; ly++) {
+                    const P u_c = su[s], u_r = su[s + 1], v_l = sv[s - 1], v_n = sv[s + EW], e_c = se[s];
+                    const P Hc = HVAR ? sH[s] : tH[ly];
+                    const P h = K::add(e_c, Hc);                        // thickness! (src/rhs.jl:131-139)
+                    const P hl = K::add(se[s - 1], HVAR ? sH[s - 1] : Hc);
+                    const P hlh = K::add(hl, h);
+                    const P hs = K::mul(q4, hlh, nz);
+                    // PV! (src/PV_advection.jl:2-18)
+                    P q = K::div(K::sub(K::add(tf[ly], K::sub(v_c, v_l)), K::sub(u_c, u_m)), K::add(hs_m, hs));
+                    if (EDGE && wwrap) {
+                        // column -1 evaluates q[end] (src/PV_advection.jl:110,126) at column N, with its own Coriolis value
+#pragma unroll
+                        for (int hh = 0; hh < V; hh++)
+                            if (cv[hh] && X[hh] == -1) {
+                                int rel = lx + hh * SHIFT + (whole ? N + 1 : -3), ha = 0;
+                                if (V == 2 && rel >= EW) { rel -= SHIFT; ha = V - 1; }
+                                const int w = ly * EW + rel;
+                                auto hv = [&](int o, int row) { return at(se, o, ha) + (HVAR ? at(sH, o, ha) : at(tH, row, 0)); };
+                                const T qt = T(0.25);
+                                const T hq = qt * (hv(w - EW - 1, ly - 1) + hv(w - EW, ly - 1)) + qt * (hv(w - 1, ly) + hv(w, ly));
+                                const T qw = (at(tf, ly, 0) + (at(sv, w, ha) - at(sv, w - 1, ha)) -
+                                              (at(su, w, ha) - at(su, w - EW, ha))) / hq;
+                                q = K::pick(K::all(qw), q, hh == 0, hh == 1);
+                            }
+                    }
+                    sq[s] = q;
+                    sU[s] = K::mulx(u_c, K::mulx(half, hlh));           // Uflux!/Vflux! (src/rhs.jl:277-304)
+                    sV[s] = K::mulx(v_c, K::mulx(half, K::add(h, h_m)));
+                    // bernoulli! (src/rhs.jl:162-180)
+                    const P KEu = K::mul(half, K::add(K::mul(u_r, u_r, nz), K::mul(u_c, u_c, nz)), nz);
+                    const P KEv = K::mul(half, K::add(K::mul(v_n, v_n, nz), K::mul(v_c, v_c, nz)), nz);
+                    sp[s] = K::add(K::mul(half, K::add(KEu, KEv), nz), K::mul(gg, e_c, nz));
+                    u_m = u_c; h_m = h; hs_m = hs; v_c = v_n;
+                    s += EW;
+                }
+            }
+        }
+        __syncthreads();
+        // ---- pass B: tendencies and the stage combination, in place
+        {
+            const int b0 = lowwall ? 0 : ay + 2, b1 = highwall ? EHv : by - 1;
+            const P a = A.a[k], b = A.b[k], o12 = A.o12;
+            if (ly0 < b1 && ly0 + R > b0) {
+                int s = ly0 * EW + lx;
+                P q_c = sq[s], q_l = sq[s - 1], q_r = sq[s + 1];
+                P V_c = sV[s], V_l = sV[s - 1];
+                P p_m = sp[s - EW];
+                P qhu_part;
+                {
+                    const P qm = sq[s - EW], qmr = sq[s - EW + 1];
+                    const P qa = K::mulx(o12, K::add(K::add(qm, q_c), q_r));
+                    const P qbr = K::mulx(o12, K::add(K::add(qmr, q_r), q_c));
+                    qhu_part = K::add(K::mul(qa, sU[s - EW], nz), K::mul(qbr, sU[s - EW + 1], nz));
+                }
+                // X, for the next stage's input, one row ahead (not used on the last stage)
+                int o = gofs(0, zy + ly0);
+                const int dX = EDGE ? X[V - 1] - X[0] : (V - 1) * SHIFT;
+                P Xu, Xv, Xe;
+                auto loadX = [&]() {
+                    Xu = K::make(A.uX[o], A.uX[o + dX]);
+                    Xv = K::make(A.vX[o], A.vX[o + dX]);
+                    Xe = K::make(A.eX[o], A.eX[o + dX]);
+                    o += g.P;
+                };
+                loadX();
+#pragma unroll
+                for (int i = 0; i < R; i++) {
+                    const int ly = ly0 + i, y = zy + ly;
+                    const P Xu_ = Xu, Xv_ = Xv, Xe_ = Xe;
+                    if (i + 1 < R) loadX();
+                    const P qn_c = sq[s + EW], qn_l = sq[s + EW - 1], qn_r = sq[s + EW + 1];
+                    const P Vn_c = sV[s + EW], Vn_l = sV[s + EW - 1];
+                    const P U_c = sU[s], U_r = sU[s + 1], p_c = sp[s], p_l = sp[s - 1];
+                    // Arakawa-Hsu combinations (src/PV_advection.jl:88-146) at column X and, for qhu, X + 1
+                    const P sc = K::add(q_c, qn_c);
+                    const P qa = K::mulx(o12, K::add(sc, qn_r));
+                    const P qb = K::mulx(o12, K::add(sc, qn_l));
+                    P qc = K::mulx(o12, K::add(K::add(q_c, q_l), qn_c));
+                    if (EDGE && wzero) {              // column 0 sums in another order
+                        const P w = K::mulx(o12, K::add(sc, q_l));
+                        qc = K::pick(w, qc, cv[0] && X[0] == 0, cv[V - 1] && X[V - 1] == 0);
+                    }
+                    const P qd = K::mulx(o12, K::add(sc, q_r));
+                    const P qbr = K::mulx(o12, K::add(K::add(q_r, qn_r), qn_c));
+                    const P qcr = K::mulx(o12, K::add(K::add(q_r, q_c), qn_r));
+                    // momentum_u! (src/rhs.jl:218-245), momentum_v! (:248-274), continuity_itself! (src/continuity.jl:52-68)
+                    const P qhv = K::add(K::add(K::add(K::mul(qa, Vn_c, nz), K::mul(qb, Vn_l, nz)), K::mul(qc, V_l, nz)),
+                                         K::mul(qd, V_c, nz));
+                    P du = K::add(K::sub(qhv, K::sub(p_c, p_l)), tFx[ly]);
+                    const P qhu = K::add(K::add(qhu_part, K::mul(qcr, U_r, nz)), K::mul(qd, U_c, nz));
+                    P dv = K::sub(tFy[ly], K::add(qhu, K::sub(p_c, p_m)));      // -(qhu + dpdy) + Fy
+                    const P ds = K::add(K::sub(U_r, U_c), K::sub(Vn_c, V_c));   // -deta
+                    qhu_part = K::add(K::mul(qa, U_c, nz), K::mul(qbr, U_r, nz));
+                    q_c = qn_c; q_l = qn_l; q_r = qn_r; V_c = Vn_c; V_l = Vn_l; p_m = p_c;
+                    if (EDGE) {
+                        // untouched halo cells go through the update with a zero tendency
+                        const bool row = y >= 0 && y < M;
+                        du = K::pick(du, K::all(T(0)), cu[0] && row, cu[V - 1] && row);
+                        if (!row || y == 0) dv = K::all(T(0));
+                    }
+                    x0u[i] = K::add(x0u[i], K::mul(a, du, nz));                 // axb!
+                    x0v[i] = K::add(x0v[i], K::mul(a, dv, nz));
+                    x0e[i] = K::sub(x0e[i], K::mul(a, ds, nz));
+                    P nu = K::add(Xu_, K::mul(b, du, nz));                       // caxb!
+                    P nv = K::add(Xv_, K::mul(b, dv, nz));
+                    P ne = K::sub(Xe_, K::mul(b, ds, nz));
+                    if (last) { nu = x0u[i]; nv = x0v[i]; ne = x0e[i]; }
+                    store(su, s, nu);
+                    store(sv, s, nv);
+                    store(se, s, ne);
+                    s += EW;
+                }
+            }
+        }
+        __syncthreads();
+        if (EDGE) {
+            ghosts();
+            __syncthreads();
+        }
+    }
+
+    // ---- tail.  T1: ν (sq), Lu (sU), Lv (sV), sqrt(KE) (sp) on the tile and one point around it
+    const bool quad = A.drag == SW_DRAG_QUADRATIC, smag = A.smag != 0;
+    if (A.tail) {
+        const int r0 = max(ly0, max(ys - 1 - zy, lowwall ? 1 : 0)), r1 = min(ly0 + R, ye + 1 - zy);
+        if (r0 < r1) {
+            const P cS = A.cSmag;
+            int s = r0 * EW + lx;
+            P u_m = su[s - EW], v_m = sv[s - EW];
+            P u_c = su[s], u_r = su[s + 1], v_c = sv[s], v_l = sv[s - 1], v_r = sv[s + 1];
+            P DS;                                          // q4 * (DSq at corners (X, y) and (X + 1, y))
+            {
+                const P d = K::add(K::sub(u_c, u_m), K::sub(v_c, v_l));
+                const P f = K::add(K::sub(u_r, su[s - EW + 1]), K::sub(v_r, v_c));
+                DS = K::mul(q4, K::add(K::mul(d, d, nz), K::mul(f, f, nz)), nz);
+            }
+#pragma unroll 2
+            for (int ly = r0; ly < r1; ly++) {
+                const P u_n = su[s + EW], un_r = su[s + EW + 1], v_n = sv[s + EW], vn_l = sv[s + EW - 1],
+                        vn_r = sv[s + EW + 1], u_l = su[s - 1];
+                // ∇²! (src/gradients.jl:29-42)
+                sU[s] = K::add(K::add(K::sub(u_l, u_c), K::sub(u_r, u_c)), K::add(K::sub(u_m, u_c), K::sub(u_n, u_c)));
+                sV[s] = K::add(K::add(K::sub(v_l, v_c), K::sub(v_r, v_c)), K::add(K::sub(v_m, v_c), K::sub(v_n, v_c)));
+                if (smag) {                                // smagorinsky_coeff! (src/diffusion.jl:68-111)
+                    const P d = K::add(K::sub(u_n, u_c), K::sub(v_n, vn_l));
+                    const P f = K::add(K::sub(un_r, u_r), K::sub(vn_r, v_n));
+                    const P DSn = K::mul(q4, K::add(K::mul(d, d, nz), K::mul(f, f, nz)), nz);
+                    const P t = K::add(K::sub(u_r, u_c), K::sub(v_n, v_c));
+                    sq[s] = K::mulx(cS, K::root(K::add(K::add(DS, DSn), K::mul(t, t, nz))));
+                    DS = DSn;
+                }
+                if (quad) {                                // bottom_drag_quadratic! (src/bottom_drag.jl:20-76)
+                    const P KEu = K::mul(half, K::add(K::mul(u_r, u_r, nz), K::mul(u_c, u_c, nz)), nz);
+                    const P KEv = K::mul(half, K::add(K::mul(v_n, v_n, nz), K::mul(v_c, v_c, nz)), nz);
+                    sp[s] = K::root(K::add(KEu, KEv));
+                }
+                u_m = u_c; u_c = u_n; u_r = un_r;
+                v_m = v_c; v_c = v_n; v_l = vn_l; v_r = vn_r;
+                s += EW;
+            }
+        }
+        __syncthreads();
+    }
+    // ---- T2: the new u, v, eta of the tile (and its untouched halo cells)
+    {
+        const int t0 = ys == 0 ? -2 : ys, t1 = ye == M ? M + 2 : ye;
+        const int r0 = max(ly0, t0 - zy), r1 = min(ly0 + R, t1 - zy);
+        if (r0 < r1) {
+            const P cD = A.cD, rD = A.rD, Dt = A.Dt_diff, nuB = A.nuB;
+            int s = r0 * EW + lx;
+            P nq_c = nuB, nq_r = nuB, S12_c = nuB, S22_m = nuB, sK_m = nuB, h_m = nuB;
+            if (A.tail) {
+                P n_m = nuB;
+                if (smag) {
+                    n_m = sq[s - EW];
+                    const P nl = sq[s - 1], nc = sq[s], nr = sq[s + 1];
+                    nq_c = K::add(K::mul(q4, K::add(sq[s - EW - 1], n_m), nz), K::mul(q4, K::add(nl, nc), nz));
+                    nq_r = K::add(K::mul(q4, K::add(n_m, sq[s - EW + 1]), nz), K::mul(q4, K::add(nc, nr), nz));
+                }
+                S22_m = K::mul(n_m, K::sub(sV[s], sV[s - EW]), nz);
+                S12_c = K::mul(nq_c, K::sub(sU[s], sU[s - EW]), nz);
+                if (quad) {
+                    sK_m = sp[s - EW];
+                    h_m = K::add(se[s - EW], HVAR ? sH[s - EW] : tH[max(r0 - 1, 0)]);
+                }
+            }
+#pragma unroll 2
+            for (int ly = r0; ly < r1; ly++) {
+                const int y = zy + ly;
+                const P u_c = su[s], v_c = sv[s];
+                P nu = u_c, nv = v_c;
+                if (A.tail) {
+                    const P Lu_l = sU[s - 1], Lu_c = sU[s], Lu_r = sU[s + 1], Lu_n = sU[s + EW];
+                    const P Lv_l = sV[s - 1], Lv_c = sV[s], Lv_r = sV[s + 1], Lv_n = sV[s + EW];
+                    P n_l = nuB, n_c = nuB, nqn_c = nuB, nqn_r = nuB;
+                    if (smag) {
+                        n_l = sq[s - 1]; n_c = sq[s];
+                        const P n_r = sq[s + 1];
+                        const P nnl = sq[s + EW - 1], nnc = sq[s + EW], nnr = sq[s + EW + 1];
+                        nqn_c = K::add(K::mul(q4, K::add(n_l, n_c), nz), K::mul(q4, K::add(nnl, nnc), nz));
+                        nqn_r = K::add(K::mul(q4, K::add(n_c, n_r), nz), K::mul(q4, K::add(nnc, nnr), nz));
+                    }
+                    P Bu = K::all(T(0)), Bv = Bu;
+                    if (quad) {
+                        const P Hc = HVAR ? sH[s] : tH[ly];
+                        const P h = K::add(se[s], Hc), hl = K::add(se[s - 1], HVAR ? sH[s - 1] : Hc);
+                        const P sK = sp[s];
+                        Bu = K::div(K::mulx(K::mulx(cD, K::mulx(half, K::add(sK, sp[s - 1]))), u_c),
+                                    K::mulx(half, K::add(h, hl)));
+                        Bv = K::div(K::mulx(K::mulx(cD, K::mulx(half, K::add(sK, sK_m))), v_c),
+                                    K::mulx(half, K::add(h, h_m)));
+                        h_m = h; sK_m = sK;
+                    } else if (A.drag == SW_DRAG_LINEAR) {
+                        Bu = K::mul(rD, u_c, nz);
+                        Bv = K::mul(rD, v_c, nz);
+                    }
+                    const P LLu1 = K::sub(K::mul(n_c, K::sub(Lu_r, Lu_c), nz), K::mul(n_l, K::sub(Lu_c, Lu_l), nz));
+                    const P S12_n = K::mul(nqn_c, K::sub(Lu_n, Lu_c), nz);
+                    const P LLu2 = K::sub(S12_n, S12_c);
+                    const P LLv1 = K::sub(K::mul(nq_r, K::sub(Lv_r, Lv_c), nz), K::mul(nq_c, K::sub(Lv_c, Lv_l), nz));
+                    const P S22 = K::mul(n_c, K::sub(Lv_n, Lv_c), nz);
+                    const P LLv2 = K::sub(S22, S22_m);
+                    nu = K::add(u_c, K::mul(Dt, K::add(K::add(Bu, LLu1), LLu2), nz));
+                    nv = K::add(v_c, K::mul(Dt, K::add(K::add(Bv, LLv1), LLv2), nz));
+                    S12_c = S12_n; S22_m = S22; nq_c = nqn_c; nq_r = nqn_r;
+                }
+                if (!EDGE) {
+                    const P ne = se[s];
+                    const int o = gofs(0, y);
+                    if (own[0]) {
+                        A.uo[o] = K::template get<0>(nu);
+                        A.vo[o] = K::template get<0>(nv);
+                        A.eo[o] = K::template get<0>(ne);
+                    }
+                    if (V == 2 && own[V - 1]) {
+                        A.uo[o + SHIFT] = K::template get<V - 1>(nu);
+                        A.vo[o + SHIFT] = K::template get<V - 1>(nv);
+                        A.eo[o + SHIFT] = K::template get<V - 1>(ne);
+                    }
+                } else {
+                    // into shared memory, for the ghost points; untouched halo cells keep their value
+                    const bool row = y >= 0 && y < M;
+                    su[s] = K::pick(nu, u_c, cu[0] && row, cu[V - 1] && row);
+                    if (row && y >= 1) sv[s] = nv;
+                }
+                s += EW;
+            }
+        }
+    }
+    if (EDGE) {
+        __syncthreads();
+        ghosts();
+        __syncthreads();
+        // the tile's outputs, the untouched columns beside them (nonperiodic u) and the ghosts copied from them
+        const int t0 = ys == 0 ? -2 : ys, t1 = ye == M ? M + 2 : ye;
+        for (int h = 0; h < V; h++) {
+            const int rel = lx + h * SHIFT;
+            bool wr = rel >= xs - zx && rel < xe - zx;
+            if (X[h] < 0 || X[h] >= N) {
+                if (per) {
+                    const int src = rel + (X[h] < 0 ? (whole ? N : -4) : (whole ? -N : 4));
+                    wr = src >= xs - zx && src < xe - zx;
+                } else {
+                    wr = X[h] < 0 ? xs == 0 : xe == N;
+                }
+            }
+            wr = wr && cv[h] && (V == 1 || (h == 0 ? lx <= EW - 3 : lx >= 2));
+            if (!wr) continue;
+            for (int y = max(zy + ly0, t0); y < min(zy + ly0 + R, t1); y++) {
+                const int s = (y - zy) * EW + lx, o = gofs(h, y);
+                if (per || X[h] >= -1) A.uo[o] = at(su, s, h);
+                if (y >= -1) A.vo[o] = at(sv, s, h);
+                if (X[h] >= -1 && X[h] <= N && y >= -1 && y <= M) A.eo[o] = at(se, s, h);
+            }
+        }
+    }
+}
+
+template <class T, class SH, bool HVAR>
+__global__ void __launch_bounds__(SH::NW * 32, 1) rk_step_kernel(const __grid_constant__ StepArgs<T> A) {
+    extern __shared__ __align__(16) unsigned char step_smem[];
+    if (A.st->stop) return;
+    const Geom& g = A.g;
+    const bool whole = A.ntx == 1 && g.N + 4 <= SH::COLS;
+    int xs, xe, zx, ys, ye, zy, zy1;
+    step_cols(g.N, g.ep, A.ntx, whole, (int)blockIdx.x % A.ntx, xs, xe, zx);
+    step_rows(g.M, A.nty, (int)blockIdx.x / A.ntx, ys, ye, zy, zy1);
+    auto* sm = reinterpret_cast<typename Pack<T>::P*>(step_smem);
+    const bool edge = zx < 2 || zx + SH::COLS > g.N - 2 || zy < 2 || zy1 > g.M - 2;
+    if (edge) step_tile<T, SH, HVAR, true>(A, sm, xs, xe, zx, ys, ye, zy, zy1, whole);
+    else step_tile<T, SH, HVAR, false>(A, sm, xs, xe, zx, ys, ye, zy, zy1, false);
+}
+
+}  // namespace swb
