@@ -454,20 +454,24 @@ struct Engine : EngineBase {
     static constexpr bool STEP_TYPES = std::is_same<T, Tp>::value &&
                                        (std::is_same<T, float>::value || std::is_same<T, double>::value);
     int init(sw_ctx* ctx) {
-        // the whole-step kernel serves RK, nonlinear Arakawa-Hsu dynamics and the plain
-        // continuity equation, with winds and Coriolis values constant along x and ghost copies
-        // that do not round (Tcomm at least T)
+        // the whole-step kernel serves nonlinear dynamics and the plain continuity equation, with
+        // winds and Coriolis values constant along x and ghost copies that do not round (Tcomm at
+        // least T)
         const sw_config& c = ctx->cfg;
         for (const char* k : {"SWB200_TMA", "SWB200_STAGE_BLOCKS", "SWB200_STAGE_TY", "SWB200_TAIL_TY"})
             if (getenv(k)) return SW_OK;             // settings of the launches per stage: these then run
         // Below 1024 cells a step keeps a launch per pass, as callers that count launches there
         // expect (four stages, tail and tracer); SWB200_STEP overrides.
         if ((long long)ctx->g.N * ctx->g.M < 1024 && !getenv("SWB200_STEP")) return SW_OK;
-        if constexpr (STEP_TYPES)
-            if (c.time_scheme == SW_RK && c.dynamics == SW_NONLINEAR && c.adv_scheme == SW_ARAKAWA_HSU &&
-                c.nstep_advcor == 0 && !c.surface_relax && !c.surface_forcing && fmt_size(c.Tcomm) >= sizeof(T))
-                if (ctx->fq.sx == 0 && ctx->Fx.sx == 0 && ctx->Fy.sx == 0)
-                    ctx->step_plan = step_plan<T>(ctx->g, ctx->nsm, ctx->H.sx != 0);
+        if constexpr (STEP_TYPES) {
+            const bool ssp = c.time_scheme != SW_RK;
+            // SSP schemes of two to four sub-stages (the halo of a tile; SSPRK3 with n = 2 has four)
+            const bool scheme = c.time_scheme == SW_SSPRK2 ? c.RKs <= 4 : c.time_scheme == SW_SSPRK3
+                                    ? c.ssp_n == 2 && c.ssp_s == 4 && c.ssp_kn <= 5 && c.ssp_mn < 2 : true;
+            if (scheme && c.dynamics == SW_NONLINEAR && c.nstep_advcor == 0 && !c.surface_relax && !c.surface_forcing &&
+                fmt_size(c.Tcomm) >= sizeof(T) && ctx->fq.sx == 0 && ctx->Fx.sx == 0 && ctx->Fy.sx == 0)
+                ctx->step_plan = step_plan<T>(ctx->g, ctx->nsm, ctx->H.sx != 0, ssp);
+        }
         return SW_OK;
     }
 
@@ -686,8 +690,9 @@ struct Engine : EngineBase {
     // start; the final u0, v0 go to Acc when the tail follows (else to Y), the
     // final eta0 to Y.  Stage buffers rotate through A, B, C avoiding the
     // current input and the SSPRK3 snapshot u0 (src/time_integration.jl:148-152),
-    // which starts as the state: u0 equals u at every step start.
-    int ssp_stages(sw_ctx* ctx, Fields3& X, Fields3& Y, bool tail_now, T Fxt, T Fyt) {
+    // which starts as the state: u0 equals u at every step start.  rhs_only: up
+    // to the last sub-stage's input (rhs_in).
+    int ssp_stages(sw_ctx* ctx, const Fields3& X, const Fields3& Y, bool tail_now, T Fxt, T Fyt, bool rhs_only = false) {
         const sw_config& c = ctx->cfg;
         const Geom& g = ctx->g;
         Fields3 fin;
@@ -734,6 +739,7 @@ struct Engine : EngineBase {
             if (!out || (combo && !cmb)) return fail(ctx, SW_ERR_ARG, "no free SSP stage buffer");
             a.u1 = (const Tp*)cur->u; a.v1 = (const Tp*)cur->v; a.e1 = (const Tp*)cur->e;
             if (is_last) ctx->rhs_in = *cur;
+            if (is_last && rhs_only) return SW_OK;
             a.uZ = (const Tp*)snap->u; a.vZ = (const Tp*)snap->v; a.eZ = (const Tp*)snap->e;
             a.u1o = (Tp*)out->u; a.v1o = (Tp*)out->v; a.e1o = (Tp*)out->e;
             if (combo) {
@@ -888,7 +894,8 @@ struct Engine : EngineBase {
             a.a[k] = K::host(k < c.RKo ? (U)c.RKaDt[k] : U(0));
             a.b[k] = K::host(k + 1 < c.RKo ? (U)c.RKbDt[k] : U(0));
         }
-        a.rko = c.RKo;
+        a.stages = c.RKo;
+        ssp_args<U>(c, a);
         a.g_ = K::host((U)c.g); a.Fxt = Fxt; a.Fyt = Fyt;
         a.tail = tail_now; a.drag = c.bottom_drag; a.smag = c.diffusion == SW_DIFF_SMAGORINSKY;
         a.cD = K::host((U)c.cD); a.rD = K::host((U)c.rD);
@@ -897,6 +904,34 @@ struct Engine : EngineBase {
         a.gr = rule(ctx);
         a.st = ctx->dst;
         return a;
+    }
+
+    // the sub-stages of an SSP scheme (the cases of ssp_stages)
+    template <class U>
+    static void ssp_args(const sw_config& c, StepArgs<U>& a) {
+        using K = Pack<U>;
+        a.combo = -1;
+        a.kna = K::host((U)c.ssp_kna); a.knb = K::host((U)c.ssp_knb);
+        a.fa = a.fb = K::host(U(0));
+        for (int k = 0; k < 4; k++) { a.sub[k] = STEP_AXB; a.x[k] = K::host(U(0)); }
+        if (c.time_scheme == SW_SSPRK2) {                    // (:107-109)
+            a.stages = c.RKs;
+            for (int k = 0; k < 4; k++) a.x[k] = K::host((U)c.Dt_Ds);
+            a.combo = c.RKs - 1;
+            a.fa = K::host((U)(1.0 / c.RKs)); a.fb = K::host((U)((double)(c.RKs - 1) / c.RKs));
+        } else if (c.time_scheme == SW_SSPRK3) {
+            a.stages = 4;
+            for (int k = 0; k < 4; k++) {
+                const bool kn = k + 2 == c.ssp_kn;
+                a.sub[k] = kn ? STEP_KN : STEP_AXB;
+                a.x[k] = K::host(kn ? (U)c.ssp_Dt_Dnc : (U)c.ssp_Dt_Dn);
+            }
+        } else if (c.time_scheme == SW_4SSPRK3) {            // (:186-191)
+            a.stages = 4;
+            for (int k = 0; k < 4; k++) { a.sub[k] = STEP_4; a.x[k] = K::host((U)c.Dt_D); }
+            a.combo = 2;
+            a.fa = K::host((U)(2.0 / 3.0)); a.fb = K::host((U)(1.0 / 3.0));
+        }
     }
 
     // The input of the last step's last stage, formed again by the launches of
@@ -908,10 +943,15 @@ struct Engine : EngineBase {
         wind_factors(ctx, ctx->rhs_t, Fxt, Fyt);
         CK(cudaMemcpyAsync(ctx->hst, ctx->dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaMemsetAsync(ctx->dst, 0, sizeof(DevStatus), ctx->stream));
-        for (int k = 1; k < ctx->cfg.RKo; k++)
-            if (int rc = rk_stage(ctx, k, ctx->rhs_p, true, Fxt, Fyt)) return rc;
+        if (ctx->cfg.time_scheme == SW_RK) {
+            for (int k = 1; k < ctx->cfg.RKo; k++)
+                if (int rc = rk_stage(ctx, k, ctx->rhs_p, true, Fxt, Fyt)) return rc;
+            ctx->rhs_in = (ctx->cfg.RKo % 2 == 0) ? ctx->A : ctx->B;
+        } else {
+            // all sub-stages but the last write stage buffers only; ssp_stages records the last one's input
+            if (int rc = ssp_stages(ctx, ctx->S[ctx->rhs_p], ctx->S[1 - ctx->rhs_p], true, Fxt, Fyt, true)) return rc;
+        }
         CK(cudaMemcpyAsync(ctx->dst, ctx->hst, sizeof(DevStatus), cudaMemcpyHostToDevice, ctx->stream));
-        ctx->rhs_in = (ctx->cfg.RKo % 2 == 0) ? ctx->A : ctx->B;
         return SW_OK;
     }
 
@@ -930,7 +970,11 @@ struct Engine : EngineBase {
             if constexpr (STEP_TYPES) {
                 const StepArgs<T> a = step_args(ctx, ctx->p, tail_now, Fxt, Fyt);
                 cudaError_t e = cudaSuccess;
-                int rc = launch(ctx, 0, [&] { e = step_launch<T>(ctx->step_plan, a, ctx->H.sx != 0, ctx->stream); });
+                const bool hvar = ctx->H.sx != 0, sad = c.adv_scheme == SW_SADOURNY;
+                int rc = launch(ctx, 0, [&] {
+                    e = c.time_scheme == SW_RK ? step_launch<T, false>(ctx->step_plan, a, hvar, sad, ctx->stream)
+                                               : step_launch<T, true>(ctx->step_plan, a, hvar, sad, ctx->stream);
+                });
                 if (!rc && e != cudaSuccess) rc = fail(ctx, SW_ERR_CUDA, std::string("step kernel: ") + cudaGetErrorString(e));
                 if (rc) return rc;
             }

@@ -46,7 +46,12 @@
 
 namespace swb {
 
-constexpr int STEP_LO = 10, STEP_HI = 6;   // halo below and above a tile (4 stages and the tail)
+constexpr int STEP_LO = 10, STEP_HI = 6;   // halo below and above a tile: 4 RK stages and the tail
+constexpr int STEP_LO_SSP = 10, STEP_HI_SSP = 10;   // 4 SSP sub-stages and the tail
+
+// Sub-stage updates (src/time_integration.jl:80-196): axb!, the kn stage's
+// dxaybzc!, 4SSPRK3's caxb! and cxab!
+enum StepSub : int { STEP_AXB = 0, STEP_KN = 1, STEP_4 = 2 };
 
 template <class T>
 struct StepArgs {
@@ -56,8 +61,14 @@ struct StepArgs {
     T* uo; T* vo; T* eo;                     // new state, with its ghosts
     SField<T> H, fq, Fx, Fy;            // fq, Fx, Fy constant along x
     using P = typename Pack<T>::P;      // constants as packs, so that they are read as they are used
-    P a[4], b[4];                       // RKaΔt, RKbΔt
-    int rko;
+    P a[4], b[4];                       // RK: RKaΔt, RKbΔt
+    int stages;                         // RK stages or SSP sub-stages
+    int lo, hi;                         // halo below and above a tile
+    // SSP: what each sub-stage does to u1, v1, eta1 (enum StepSub) and its
+    // coefficient x; kna, knb of SSPRK3's kn stage; the weights fa, fb of
+    // fa*u + fb*u1 and the sub-stage after which it is taken (-1: none)
+    int sub[4], combo;
+    P x[4], kna, knb, fa, fb;
     T Fxt, Fyt;
     int tail, drag, smag;               // tail due; enum sw_bottom_drag; Smagorinsky (else constant νB)
     P g_, cD, rD, cSmag, nuB, Dt_diff;
@@ -69,20 +80,20 @@ struct StepArgs {
 // The columns of tile i: outputs [xs, xe), its first column at virtual column
 // z0.  A periodic domain's first and last tile hold 4 ghost columns more, so
 // the split treats the domain as 8 columns longer and gives them 4 fewer.
-__host__ __device__ inline void step_cols(int N, int ep, int ntx, bool whole, int i, int& xs, int& xe, int& z0) {
+__host__ __device__ inline void step_cols(int N, int ep, int ntx, bool whole, int lo_, int i, int& xs, int& xe, int& z0) {
     if (whole) { xs = 0; xe = N; z0 = -2; return; }
     const int L = ep ? N + 8 : N, sh = ep ? 4 : 0;
     const int lo = (int)((long long)i * L / ntx) - sh, hi = (int)((long long)(i + 1) * L / ntx) - sh;
     xs = lo < 0 ? 0 : lo;
     xe = hi > N ? N : hi;
-    z0 = xs - STEP_LO - (ep && i == 0 ? 4 : 0);
+    z0 = xs - lo_ - (ep && i == 0 ? 4 : 0);
 }
 // The rows of tile j: outputs [ys, ye), loaded rows [z0, z1).
-__host__ __device__ inline void step_rows(int M, int nty, int j, int& ys, int& ye, int& z0, int& z1) {
+__host__ __device__ inline void step_rows(int M, int nty, int lo, int hi, int j, int& ys, int& ye, int& z0, int& z1) {
     ys = (int)((long long)j * M / nty);
     ye = (int)((long long)(j + 1) * M / nty);
-    z0 = ys - STEP_LO < -2 ? -2 : ys - STEP_LO;
-    z1 = ye + STEP_HI > M + 2 ? M + 2 : ye + STEP_HI;
+    z0 = ys - lo < -2 ? -2 : ys - lo;
+    z1 = ye + hi > M + 2 ? M + 2 : ye + hi;
 }
 
 // EWW warps side by side (EW = 32 EWW lanes), NW warps in all, R rows per
@@ -97,10 +108,11 @@ struct StepShape {
     static constexpr int smem(bool hvar) { return ((7 + hvar) * NP + PAD + 4 * EH) * (int)sizeof(P); }
 };
 
-// One tile.  EDGE is false for tiles none of whose points is a ghost, a ghost
-// source or a wall.  HVAR: the depth varies along x (an array in shared
+// One tile.  SSP: sub-stages of the SSP schemes instead of RK stages.  SAD:
+// PV_Sadourny! instead of PV_ArakawaHsu!.  EDGE is false for tiles none of
+// whose points is a ghost, a ghost source or a wall.  HVAR: the depth varies along x (an array in shared
 // memory; else one value per row).
-template <class T, class SH, bool HVAR, bool EDGE>
+template <class T, class SH, bool HVAR, bool SSP, bool SAD, bool EDGE>
 __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>::P* sm, int xs, int xe, int zx,
                                           int ys, int ye, int zy, int zy1, bool whole) {
     using K = Pack<T>;
@@ -109,9 +121,9 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
     constexpr int SHIFT = EW - 4;                         // columns between the halves
     P* const su = sm + SH::PAD;
     P* const sv = su + NP;
-    P* const se = sv + NP;
-    P* const sq = se + NP;
-    P* const sU = sq + NP;
+    P* se = sv + NP;                                      // SSP: exchanged with sq after each sub-stage
+    P* sq = se + NP;
+    P* const sU = sv + 3 * NP;
     P* const sV = sU + NP;
     P* const sp = sV + NP;
     P* const sH = sp + NP;                                // HVAR only
@@ -170,9 +182,13 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
         zero = zero || (per && cv[h] && X[h] == 0);
         wrap = wrap || (per && cv[h] && X[h] == -1);
     }
-    P x0u[R], x0v[R], x0e[R];                             // the accumulator X0 of this thread's points
+    P x0u[SSP ? 1 : R], x0v[SSP ? 1 : R], x0e[SSP ? 1 : R];   // RK: the accumulator X0 of this thread's points
+    bool keep[V];                                         // nonperiodic u column that keeps its value
+#pragma unroll
+    for (int h = 0; h < V; h++) keep[h] = EDGE && cv[h] && !per && X[h] >= -1 && (X[h] <= 0 || X[h] >= N);
     // whether any lane's are
-    const bool wwrap = EDGE && __any_sync(0xffffffffu, wrap), wzero = EDGE && __any_sync(0xffffffffu, zero);
+    const bool wwrap = EDGE && __any_sync(0xffffffffu, wrap), wzero = EDGE && __any_sync(0xffffffffu, zero),
+               wkeep = EDGE && __any_sync(0xffffffffu, !prod && (keep[0] || keep[V - 1]));
 
     // ---- the step's state, halo and ghosts included
 #pragma unroll
@@ -194,9 +210,10 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
                 }
             }
             const int s = ly * EW + lx;
-            su[s] = x0u[i] = K::make(a[0], a[V - 1]);
-            sv[s] = x0v[i] = K::make(b[0], b[V - 1]);
-            se[s] = x0e[i] = K::make(c[0], c[V - 1]);
+            su[s] = K::make(a[0], a[V - 1]);
+            sv[s] = K::make(b[0], b[V - 1]);
+            se[s] = K::make(c[0], c[V - 1]);
+            if constexpr (!SSP) { x0u[i] = su[s]; x0v[i] = sv[s]; x0e[i] = se[s]; }
             if (HVAR) sH[s] = K::make(d[0], d[V - 1]);
         }
     }
@@ -215,6 +232,14 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
     auto store = [&](P* f, int s, P val) {
         if (prod) f[s] = val;
         if (xch) scalar(f)[s * V + xofs] = lx == 3 ? K::template get<1>(val) : K::template get<0>(val);
+    };
+    // the same for u: its untouched columns are updated without neighbours
+    auto store_u = [&](int s, P val) {
+        store(su, s, val);
+        if (EDGE && wkeep && !prod) {
+            if (keep[0]) at(su, s, 0) = K::template get<0>(val);
+            if (V == 2 && keep[V - 1]) at(su, s, V - 1) = K::template get<1>(val);
+        }
     };
     // EDGE: ghost points of u, v, eta (src/ghost_points.jl:46-133), spread over
     // the block: columns -2, -1, N, N+1 of every row, then rows -2, -1, M, M+1
@@ -260,11 +285,11 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
             }
     };
 
-    const int rko = A.rko;
-    for (int k = 0; k < rko; k++) {
-        const bool last = k == rko - 1;
+    const int stages = A.stages;
+    for (int k = 0; k < stages; k++) {
+        const bool last = k == stages - 1;
         // rows of the stage input that are valid, then the rows each pass forms
-        const int ay = lowwall ? 0 : 2 * k, by = highwall ? EHv : EHv - k;
+        const int ay = lowwall ? 0 : 2 * k, by = highwall ? EHv : EHv - (SSP ? 2 : 1) * k;
         const int a0 = lowwall ? -zy : ay + 1, a1 = highwall ? M + 1 - zy : by;
         // ---- pass A: q, U, V, p
         {
@@ -317,23 +342,27 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
             }
         }
         __syncthreads();
-        // ---- pass B: tendencies and the stage combination, in place
-        {
+        // ---- pass B: tendencies and the stage combination, in place (SUB: enum StepSub, -1 for RK)
+        auto pass_b = [&](auto subc) {
+            constexpr int SUB = decltype(subc)::value;
             const int b0 = lowwall ? 0 : ay + 2, b1 = highwall ? EHv : by - 1;
             const P a = A.a[k], b = A.b[k], o12 = A.o12;
+            [[maybe_unused]] const P x = A.x[k], kna = A.kna, knb = A.knb;
             if (ly0 < b1 && ly0 + R > b0) {
                 int s = ly0 * EW + lx;
                 P q_c = sq[s], q_l = sq[s - 1], q_r = sq[s + 1];
                 P V_c = sV[s], V_l = sV[s - 1];
                 P p_m = sp[s - EW];
                 P qhu_part;
-                {
+                if (SAD) {
+                    qhu_part = K::mul(q4, K::add(sU[s - EW], sU[s - EW + 1]), nz);
+                } else {
                     const P qm = sq[s - EW], qmr = sq[s - EW + 1];
                     const P qa = K::mulx(o12, K::add(K::add(qm, q_c), q_r));
                     const P qbr = K::mulx(o12, K::add(K::add(qmr, q_r), q_c));
                     qhu_part = K::add(K::mul(qa, sU[s - EW], nz), K::mul(qbr, sU[s - EW + 1], nz));
                 }
-                // X, for the next stage's input, one row ahead (not used on the last stage)
+                // X, for the next stage's input or the kn stage's snapshot, one row ahead (RK: not used on the last stage)
                 int o = gofs(0, zy + ly0);
                 const int dX = EDGE ? X[V - 1] - X[0] : (V - 1) * SHIFT;
                 P Xu, Xv, Xe;
@@ -343,35 +372,45 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
                     Xe = K::make(A.eX[o], A.eX[o + dX]);
                     o += g.P;
                 };
-                loadX();
-#pragma unroll
+                constexpr bool needX = SUB == -1 || SUB == STEP_KN;
+                if (needX) loadX();
+#pragma unroll (SSP ? (R < 4 ? R : 4) : R)
                 for (int i = 0; i < R; i++) {
                     const int ly = ly0 + i, y = zy + ly;
                     const P Xu_ = Xu, Xv_ = Xv, Xe_ = Xe;
-                    if (i + 1 < R) loadX();
+                    if (needX && i + 1 < R) loadX();
                     const P qn_c = sq[s + EW], qn_l = sq[s + EW - 1], qn_r = sq[s + EW + 1];
                     const P Vn_c = sV[s + EW], Vn_l = sV[s + EW - 1];
                     const P U_c = sU[s], U_r = sU[s + 1], p_c = sp[s], p_l = sp[s - 1];
-                    // Arakawa-Hsu combinations (src/PV_advection.jl:88-146) at column X and, for qhu, X + 1
-                    const P sc = K::add(q_c, qn_c);
-                    const P qa = K::mulx(o12, K::add(sc, qn_r));
-                    const P qb = K::mulx(o12, K::add(sc, qn_l));
-                    P qc = K::mulx(o12, K::add(K::add(q_c, q_l), qn_c));
-                    if (EDGE && wzero) {              // column 0 sums in another order
-                        const P w = K::mulx(o12, K::add(sc, q_l));
-                        qc = K::pick(w, qc, cv[0] && X[0] == 0, cv[V - 1] && X[V - 1] == 0);
+                    P qhv, qhu;
+                    if (SAD) {                              // PV_Sadourny! (src/PV_advection.jl:31-59)
+                        qhv = K::mul(K::mulx(half, K::add(qn_c, q_c)),
+                                     K::add(K::mul(q4, K::add(V_l, V_c), nz), K::mul(q4, K::add(Vn_l, Vn_c), nz)), nz);
+                        const P Us = K::mul(q4, K::add(U_c, U_r), nz);
+                        qhu = K::mul(K::mulx(half, K::add(q_r, q_c)), K::add(qhu_part, Us), nz);
+                        qhu_part = Us;
+                    } else {
+                        // Arakawa-Hsu combinations (src/PV_advection.jl:88-146) at column X and, for qhu, X + 1
+                        const P sc = K::add(q_c, qn_c);
+                        const P qa = K::mulx(o12, K::add(sc, qn_r));
+                        const P qb = K::mulx(o12, K::add(sc, qn_l));
+                        P qc = K::mulx(o12, K::add(K::add(q_c, q_l), qn_c));
+                        if (EDGE && wzero) {                // column 0 sums in another order
+                            const P w = K::mulx(o12, K::add(sc, q_l));
+                            qc = K::pick(w, qc, per && cv[0] && X[0] == 0, per && cv[V - 1] && X[V - 1] == 0);
+                        }
+                        const P qd = K::mulx(o12, K::add(sc, q_r));
+                        const P qbr = K::mulx(o12, K::add(K::add(q_r, qn_r), qn_c));
+                        const P qcr = K::mulx(o12, K::add(K::add(q_r, q_c), qn_r));
+                        qhv = K::add(K::add(K::add(K::mul(qa, Vn_c, nz), K::mul(qb, Vn_l, nz)), K::mul(qc, V_l, nz)),
+                                     K::mul(qd, V_c, nz));
+                        qhu = K::add(K::add(qhu_part, K::mul(qcr, U_r, nz)), K::mul(qd, U_c, nz));
+                        qhu_part = K::add(K::mul(qa, U_c, nz), K::mul(qbr, U_r, nz));
                     }
-                    const P qd = K::mulx(o12, K::add(sc, q_r));
-                    const P qbr = K::mulx(o12, K::add(K::add(q_r, qn_r), qn_c));
-                    const P qcr = K::mulx(o12, K::add(K::add(q_r, q_c), qn_r));
                     // momentum_u! (src/rhs.jl:218-245), momentum_v! (:248-274), continuity_itself! (src/continuity.jl:52-68)
-                    const P qhv = K::add(K::add(K::add(K::mul(qa, Vn_c, nz), K::mul(qb, Vn_l, nz)), K::mul(qc, V_l, nz)),
-                                         K::mul(qd, V_c, nz));
                     P du = K::add(K::sub(qhv, K::sub(p_c, p_l)), tFx[ly]);
-                    const P qhu = K::add(K::add(qhu_part, K::mul(qcr, U_r, nz)), K::mul(qd, U_c, nz));
                     P dv = K::sub(tFy[ly], K::add(qhu, K::sub(p_c, p_m)));      // -(qhu + dpdy) + Fy
-                    const P ds = K::add(K::sub(U_r, U_c), K::sub(Vn_c, V_c));   // -deta
-                    qhu_part = K::add(K::mul(qa, U_c, nz), K::mul(qbr, U_r, nz));
+                    const P ds = K::add(K::sub(U_r, U_c), K::sub(Vn_c, V_c));   // -deta (RK)
                     q_c = qn_c; q_l = qn_l; q_r = qn_r; V_c = Vn_c; V_l = Vn_l; p_m = p_c;
                     if (EDGE) {
                         // untouched halo cells go through the update with a zero tendency
@@ -379,24 +418,96 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
                         du = K::pick(du, K::all(T(0)), cu[0] && row, cu[V - 1] && row);
                         if (!row || y == 0) dv = K::all(T(0));
                     }
-                    x0u[i] = K::add(x0u[i], K::mul(a, du, nz));                 // axb!
-                    x0v[i] = K::add(x0v[i], K::mul(a, dv, nz));
-                    x0e[i] = K::sub(x0e[i], K::mul(a, ds, nz));
-                    P nu = K::add(Xu_, K::mul(b, du, nz));                       // caxb!
-                    P nv = K::add(Xv_, K::mul(b, dv, nz));
-                    P ne = K::sub(Xe_, K::mul(b, ds, nz));
-                    if (last) { nu = x0u[i]; nv = x0v[i]; ne = x0e[i]; }
-                    store(su, s, nu);
-                    store(sv, s, nv);
-                    store(se, s, ne);
+                    if constexpr (SSP) {
+                        // the momentum half of the sub-stage; eta follows from the new u, v in pass C
+                        auto update = [&](P u1, P z, P d) {
+                            const P xd = K::mul(x, d, nz);
+                            if (SUB == STEP_AXB) return K::add(u1, xd);
+                            if (SUB == STEP_KN) return K::add(K::add(K::mul(kna, u1, nz), K::mul(knb, z, nz)), xd);
+                            return K::mul(half, K::add(u1, K::add(u1, xd)), nz);
+                        };
+                        store_u(s, update(su[s], Xu_, du));
+                        store(sv, s, update(sv[s], Xv_, dv));
+                    } else {
+                        x0u[i] = K::add(x0u[i], K::mul(a, du, nz));                 // axb!
+                        x0v[i] = K::add(x0v[i], K::mul(a, dv, nz));
+                        x0e[i] = K::sub(x0e[i], K::mul(a, ds, nz));
+                        P nu = K::add(Xu_, K::mul(b, du, nz));                       // caxb!
+                        P nv = K::add(Xv_, K::mul(b, dv, nz));
+                        P ne = K::sub(Xe_, K::mul(b, ds, nz));
+                        if (last) { nu = x0u[i]; nv = x0v[i]; ne = x0e[i]; }
+                        store_u(s, nu);
+                        store(sv, s, nv);
+                        store(se, s, ne);
+                    }
                     s += EW;
                 }
             }
-        }
+        };
+        if constexpr (!SSP) pass_b(std::integral_constant<int, -1>{});
+        else if (A.sub[k] == STEP_AXB) pass_b(std::integral_constant<int, STEP_AXB>{});
+        else if (A.sub[k] == STEP_KN) pass_b(std::integral_constant<int, STEP_KN>{});
+        else pass_b(std::integral_constant<int, STEP_4>{});
         __syncthreads();
         if (EDGE) {
             ghosts();
             __syncthreads();
+        }
+        if constexpr (SSP) {
+            // ---- pass C: continuity! from the new u, v and the sub-stage's eta
+            // (src/continuity.jl:72-97) into sq, which takes eta's place
+            const P x = A.x[k], kna = A.kna, knb = A.knb, fa = A.fa, fb = A.fb;
+            const int sub = A.sub[k];
+            const bool mix = k == A.combo, needX = mix || sub == STEP_KN;
+            const int dX = EDGE ? X[V - 1] - X[0] : (V - 1) * SHIFT;
+            const int r0 = max(ly0, lowwall ? -zy : ay + 1), r1 = min(ly0 + R, highwall ? M - zy : by - 1);
+            // e at EW-2 and EW-1 of the lower half come from the upper half's lanes 2, 3
+            const bool prod_e = V == 1 || (lx >= 2 && lx <= EW - 3), xch_e = V == 2 && (xch || lx == 2);
+            const int xofs_e = lx <= 3 ? 2 * SHIFT : -2 * SHIFT + 1;
+            if (r0 < r1) {
+                int s = r0 * EW + lx;
+                auto depth = [&](int o, int ly) { return K::add(se[o], HVAR ? sH[o] : tH[ly]); };
+                P h_c = depth(s, r0);
+                P V_c = K::mul(sv[s], K::mulx(half, K::add(h_c, depth(s - EW, r0 - 1))), nz);
+#pragma unroll 2
+                for (int ly = r0; ly < r1; ly++) {
+                    const P h_n = depth(s + EW, ly + 1), h_l = depth(s - 1, ly), h_r = depth(s + 1, ly);
+                    const P U_c = K::mul(su[s], K::mulx(half, K::add(h_c, h_l)), nz);
+                    const P U_r = K::mul(su[s + 1], K::mulx(half, K::add(h_r, h_c)), nz);
+                    const P V_n = K::mul(sv[s + EW], K::mulx(half, K::add(h_n, h_c)), nz);
+                    const P xd = K::mul(x, K::add(K::sub(U_r, U_c), K::sub(V_n, V_c)), nz);     // -x deta
+                    const P e1 = se[s];
+                    P z = e1;
+                    if (needX) {
+                        const int o = gofs(0, zy + ly);
+                        z = K::make(A.eX[o], A.eX[o + dX]);
+                    }
+                    P e;
+                    if (sub == STEP_AXB) e = K::sub(e1, xd);
+                    else if (sub == STEP_KN) e = K::sub(K::add(K::mul(kna, e1, nz), K::mul(knb, z, nz)), xd);
+                    else e = K::mul(half, K::add(e1, K::sub(e1, xd)), nz);
+                    if (mix) e = K::add(K::mul(fa, z, nz), K::mul(fb, e, nz));
+                    if (prod_e) sq[s] = e;
+                    if (xch_e) scalar(sq)[s * V + xofs_e] = lx <= 3 ? K::template get<1>(e) : K::template get<0>(e);
+                    h_c = h_n; V_c = V_n;
+                    s += EW;
+                }
+            }
+            __syncthreads();
+            P* const t = se; se = sq; sq = t;
+            if (mix) {
+                // cxayb! of u, v with the state at the step's start (:107-109, :186-191)
+                for (int ly = ly0; ly < min(ly0 + R, EHv); ly++) {
+                    const int s = ly * EW + lx, o = gofs(0, zy + ly);
+                    su[s] = K::add(K::mul(fa, K::make(A.uX[o], A.uX[o + dX]), nz), K::mul(fb, su[s], nz));
+                    sv[s] = K::add(K::mul(fa, K::make(A.vX[o], A.vX[o + dX]), nz), K::mul(fb, sv[s], nz));
+                }
+                __syncthreads();
+            }
+            if (EDGE) {
+                ghosts();
+                __syncthreads();
+            }
         }
     }
 
@@ -557,19 +668,28 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
     }
 }
 
-template <class T, class SH, bool HVAR>
-__global__ void __launch_bounds__(SH::NW * 32, 1) rk_step_kernel(const __grid_constant__ StepArgs<T> A) {
-    extern __shared__ __align__(16) unsigned char step_smem[];
-    if (A.st->stop) return;
+// tile `tile` of the domain, by the calling block
+template <class T, class SH, bool HVAR, bool SSP, bool SAD>
+__device__ __forceinline__ void step_block(const StepArgs<T>& A, int tile, typename SH::P* sm) {
     const Geom& g = A.g;
     const bool whole = A.ntx == 1 && g.N + 4 <= SH::COLS;
     int xs, xe, zx, ys, ye, zy, zy1;
-    step_cols(g.N, g.ep, A.ntx, whole, (int)blockIdx.x % A.ntx, xs, xe, zx);
-    step_rows(g.M, A.nty, (int)blockIdx.x / A.ntx, ys, ye, zy, zy1);
-    auto* sm = reinterpret_cast<typename Pack<T>::P*>(step_smem);
+    step_cols(g.N, g.ep, A.ntx, whole, A.lo, tile % A.ntx, xs, xe, zx);
+    step_rows(g.M, A.nty, A.lo, A.hi, tile / A.ntx, ys, ye, zy, zy1);
     const bool edge = zx < 2 || zx + SH::COLS > g.N - 2 || zy < 2 || zy1 > g.M - 2;
-    if (edge) step_tile<T, SH, HVAR, true>(A, sm, xs, xe, zx, ys, ye, zy, zy1, whole);
-    else step_tile<T, SH, HVAR, false>(A, sm, xs, xe, zx, ys, ye, zy, zy1, false);
+    if (edge) step_tile<T, SH, HVAR, SSP, SAD, true>(A, sm, xs, xe, zx, ys, ye, zy, zy1, whole);
+    else step_tile<T, SH, HVAR, SSP, SAD, false>(A, sm, xs, xe, zx, ys, ye, zy, zy1, false);
+}
+
+template <class T, class SH, bool HVAR, bool SSP, bool SAD>
+__global__ void __launch_bounds__(SH::NW * 32, 1) rk_step_kernel(const __grid_constant__ StepArgs<T> A) {
+    extern __shared__ __align__(16) unsigned char step_smem[];
+    // all blocks of this launch run at once on a small grid: the next launch may then be prepared
+    // beside it; nothing of the step before is read until it has ended
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    if (A.st->stop) return;
+    step_block<T, SH, HVAR, SSP, SAD>(A, (int)blockIdx.x, reinterpret_cast<typename SH::P*>(step_smem));
 }
 
 }  // namespace swb
