@@ -453,25 +453,27 @@ template <class T, class Tp>
 struct Engine : EngineBase {
     static constexpr bool STEP_TYPES = std::is_same<T, Tp>::value &&
                                        (std::is_same<T, float>::value || std::is_same<T, double>::value);
+    // The whole-step kernel serves nonlinear dynamics and the plain continuity
+    // equation, with winds and Coriolis values constant along x and ghost
+    // copies that do not round (Tcomm at least T); of the SSP schemes those of
+    // two to four sub-stages (the halo of a tile; SSPRK3 with n = 2 has four).
+    static bool step_fits(const sw_ctx* ctx) {
+        const sw_config& c = ctx->cfg;
+        const bool scheme = c.time_scheme == SW_SSPRK2 ? c.RKs <= 4 : c.time_scheme == SW_SSPRK3
+                                ? c.ssp_n == 2 && c.ssp_s == 4 && c.ssp_kn <= 5 && c.ssp_mn < 2 : true;
+        return STEP_TYPES && scheme && c.dynamics == SW_NONLINEAR && c.nstep_advcor == 0 && !c.surface_relax &&
+               !c.surface_forcing && fmt_size(c.Tcomm) >= sizeof(T) && ctx->fq.sx == 0 && ctx->Fx.sx == 0 &&
+               ctx->Fy.sx == 0;
+    }
     int init(sw_ctx* ctx) {
-        // the whole-step kernel serves nonlinear dynamics and the plain continuity equation, with
-        // winds and Coriolis values constant along x and ghost copies that do not round (Tcomm at
-        // least T)
         const sw_config& c = ctx->cfg;
         for (const char* k : {"SWB200_TMA", "SWB200_STAGE_BLOCKS", "SWB200_STAGE_TY", "SWB200_TAIL_TY"})
             if (getenv(k)) return SW_OK;             // settings of the launches per stage: these then run
         // Below 1024 cells a step keeps a launch per pass, as callers that count launches there
         // expect (four stages, tail and tracer); SWB200_STEP overrides.
         if ((long long)ctx->g.N * ctx->g.M < 1024 && !getenv("SWB200_STEP")) return SW_OK;
-        if constexpr (STEP_TYPES) {
-            const bool ssp = c.time_scheme != SW_RK;
-            // SSP schemes of two to four sub-stages (the halo of a tile; SSPRK3 with n = 2 has four)
-            const bool scheme = c.time_scheme == SW_SSPRK2 ? c.RKs <= 4 : c.time_scheme == SW_SSPRK3
-                                    ? c.ssp_n == 2 && c.ssp_s == 4 && c.ssp_kn <= 5 && c.ssp_mn < 2 : true;
-            if (scheme && c.dynamics == SW_NONLINEAR && c.nstep_advcor == 0 && !c.surface_relax && !c.surface_forcing &&
-                fmt_size(c.Tcomm) >= sizeof(T) && ctx->fq.sx == 0 && ctx->Fx.sx == 0 && ctx->Fy.sx == 0)
-                ctx->step_plan = step_plan<T>(ctx->g, ctx->nsm, ctx->H.sx != 0, ssp);
-        }
+        if constexpr (STEP_TYPES)
+            if (step_fits(ctx)) ctx->step_plan = step_plan<T>(ctx->g, ctx->nsm, ctx->H.sx != 0, c.time_scheme != SW_RK);
         return SW_OK;
     }
 
@@ -1877,6 +1879,8 @@ struct BatchGroup {
     int per = 1, rko = 4, drag = 0, storage = SW_STORE_NATIVE;
     bool smag = false, um_is_u = true, cons = false, tracer_any = false;
     std::vector<int> idx;                      // member indices
+    int step_shape = -1;                       // >= 0: the whole-step kernel serves the group, with these tiles
+    std::vector<StepPlan> plans;
     // argument tables: StageArgs, TailArgs, TracerArgs, BatchCopy, BatchNan for
     // native members; S16StageArgs, S16TailBatchArgs, S16TracerBatchArgs,
     // BatchCopy16, BatchNan16 of the storage type for 16-bit members
@@ -1950,7 +1954,7 @@ int batch_tables(sw_batch* b, BatchGroup& gr) {
     const int n = (int)gr.idx.size();
     int rc;
     for (int p = 0; p < 2; p++) {
-        for (int ti = 0; ti < BATCH_NTY; ti++) {
+        for (int ti = 0; ti < BATCH_NTY && gr.step_shape < 0; ti++) {
             for (int k = 1; k <= gr.rko; k++) {
                 std::vector<StageArgs<float, float>> v;
                 for (int m : gr.idx) {
@@ -2058,8 +2062,21 @@ int batch_build(sw_batch* b) {
         }
         b->groups[it->second].idx.push_back(m);
     }
+    // strip heights asked for by the environment belong to the launches per stage
+    const char* envs = getenv("SWB200_STEP");
+    const bool steps_ok = !getenv("SWB200_BATCH_TY") && !(envs && atoi(envs) < 0);
     for (BatchGroup& gr : b->groups) {
         const int n = (int)gr.idx.size();
+        if (steps_ok && gr.storage == SW_STORE_NATIVE) {
+            std::vector<Geom> gs;
+            bool fits = true;
+            for (int m : gr.idx) {
+                gs.push_back(b->mem[m]->g);
+                fits = fits && E::step_fits(b->mem[m]) && b->mem[m]->cfg.adv_scheme == SW_ARAKAWA_HSU;
+            }
+            gr.plans.resize(n);
+            if (fits) gr.step_shape = step_batch_plan(gs.data(), n, b->mem[gr.idx[0]]->nsm, gr.plans.data());
+        }
         std::vector<int> cs[BATCH_NTY], ct[BATCH_NTY], ctr, nbx, cc, cn;
         std::vector<BatchMember> mems;
         for (int m : gr.idx) {
@@ -2130,6 +2147,23 @@ int batch_group_step(sw_batch* b, const BatchGroup& gr, int p, cudaStream_t s, i
     int launches = 0;
     const int nst = gr.n_stage[ti], ntl = gr.n_tail[ti];
     const int* bst = gr.b_stage[ti];
+    if (gr.step_shape >= 0) {
+        // stages and tail of up to STEP_BATCH members in one launch
+        std::unique_ptr<StepBatch> sb(new StepBatch());
+        for (int m0 = 0; m0 < n; m0 += STEP_BATCH) {
+            sb->n = std::min(STEP_BATCH, n - m0);
+            sb->istep = i;
+            for (int q = 0; q < sb->n; q++) {
+                sw_ctx* ctx = b->mem[gr.idx[m0 + q]];
+                sb->m[q] = dynamic_cast<Engine<float, float>*>(ctx->eng.get())->step_args(ctx, p, true, 1.f, 1.f);
+                sb->m[q].ntx = gr.plans[m0 + q].ntx;
+                sb->m[q].nty = gr.plans[m0 + q].nty;
+                sb->nt[q] = ctx->cfg.nt;
+            }
+            (void)step_batch_launch(gr.step_shape, *sb, s);    // a failure shows at the capture's end
+            launches++;
+        }
+    } else {
     for (int k = 1; k <= gr.rko; k++) {
         const auto* a = static_cast<const StageArgs<float, float>*>(gr.stage[ti][p][k - 1]);
         if (k == 1) rk_stage_batch<float, float, PER, true, false, TY><<<nst, 128, 0, s>>>(a, bst, n, gr.memb, i);
@@ -2148,6 +2182,7 @@ int batch_group_step(sw_batch* b, const BatchGroup& gr, int p, cudaStream_t s, i
         else tail(tail_batch<float, float, PER, SW_DRAG_NONE, false, TY>);
     }
     launches += gr.rko + 1;
+    }
     if (gr.tracer_any) {
         if (!gr.um_is_u) {
             copy_batch<<<gr.n_copy, 256, 0, s>>>(static_cast<const BatchCopy*>(gr.copy[p]), gr.b_copy, n, gr.memb, i);
@@ -2338,6 +2373,9 @@ int sw_batch_run(sw_batch* b, int64_t nsteps, sw_status* statuses) {
         b->launches += b->launches_per_step[ti][p];
         i++;
     };
+    // with no group left on the strip kernels there is no height to choose
+    if (std::all_of(b->groups.begin(), b->groups.end(), [](const BatchGroup& g) { return g.step_shape >= 0; }))
+        b->ty = BATCH_NTY - 1;
     if (b->ty < 0) {   // the tile height: forced, remembered for this shape, or timed now
         const char* env = getenv("SWB200_BATCH_TY");
         const int want = env ? atoi(env) : 0;
