@@ -43,6 +43,14 @@
 #include <vector>
 
 #include "swb200.h"
+#include "sw_pool.h"
+
+#ifdef SWA_HOST_CHECK   // built without the runtime; allocates on the host only
+namespace swb {
+cudaError_t pool_malloc(void** p, size_t bytes) { return cudaMalloc(p, bytes); }
+void pool_free(void* p, size_t) { cudaFree(p); }
+}  // namespace swb
+#endif
 
 namespace swa {
 
@@ -1432,7 +1440,7 @@ struct Adjoint {
     cudaStream_t s3 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     bool host = false;
-    std::vector<void*> blocks;
+    std::vector<std::pair<void*, size_t>> blocks;   // device blocks (pool_malloc) and their sizes
     cudaStream_t s = nullptr, s2 = nullptr;
     // step graphs, by whether the step ends with drag and diffusion ([1]) or not ([0])
     cudaGraphExec_t g_fwd[2] = {}, g_adj[2] = {}, g_adj_st[2] = {}, g_fwd2[2] = {};
@@ -1453,8 +1461,8 @@ struct Adjoint {
         for (int t = 0; t < 2; t++)
             for (cudaGraphExec_t g : {g_fwd[t], g_adj[t], g_adj_st[t], g_fwd2[t]})
                 if (g) cudaGraphExecDestroy(g);
-        for (void* p : blocks) {
-            if (host) std::free(p); else cudaFree(p);
+        for (auto& p : blocks) {
+            if (host) std::free(p.first); else swb::pool_free(p.first, p.second);
         }
         if (s) cudaStreamDestroy(s);
         if (s2) cudaStreamDestroy(s2);
@@ -1470,9 +1478,9 @@ struct Adjoint {
         const size_t bytes = std::max<size_t>(elems, 1) * sizeof(T);
         void* p = nullptr;
         if (host) p = std::calloc(1, bytes);
-        else if (cudaMalloc(&p, bytes) != cudaSuccess) { p = nullptr; (void)cudaGetLastError(); }
+        else if (swb::pool_malloc(&p, bytes) != cudaSuccess) { p = nullptr; (void)cudaGetLastError(); }
         if (!p) return nullptr;
-        blocks.push_back(p);
+        blocks.push_back({p, bytes});
         return static_cast<T*>(p);
     }
     cudaError_t upload(void* dst, const void* src, size_t bytes) {
@@ -1536,9 +1544,9 @@ struct Adjoint {
             const size_t total = cv.total();
             void* p = nullptr;
             if (host) p = std::calloc(total, sizeof(T));
-            else if (cudaMalloc(&p, total * sizeof(T)) != cudaSuccess) { p = nullptr; cudaGetLastError(); }
+            else if (swb::pool_malloc(&p, total * sizeof(T)) != cudaSuccess) { p = nullptr; cudaGetLastError(); }
             if (!p) continue;
-            blocks.push_back(p);
+            blocks.push_back({p, total * sizeof(T)});
             cv.place(static_cast<T*>(p));
             for (auto& x : sl) {
                 x.base = x.u.d;
@@ -1708,9 +1716,9 @@ struct Adjoint {
                     const size_t n = (size_t)nb * (size_t)nrecords * re;
                     void* p = nullptr;
                     if (host) p = std::calloc(n, sizeof(T));
-                    else if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) { p = nullptr; (void)cudaGetLastError(); }
+                    else if (swb::pool_malloc(&p, n * sizeof(T)) != cudaSuccess) { p = nullptr; (void)cudaGetLastError(); }
                     if (p) {
-                        blocks.push_back(p);
+                        blocks.push_back({p, n * sizeof(T)});
                         records = static_cast<T*>(p);
                         stored = true;
                         overlap = nb == 2;
@@ -1989,13 +1997,16 @@ int adjoint_run(bool host, const sw_config& c, const sw_static& st, const void* 
     // the J row sums are allocated before the checkpoint slots, which take the
     // largest block that fits and would otherwise leave no room for them
     double* rowsum = host ? static_cast<double*>(std::calloc(w.ny, sizeof(double))) : nullptr;
-    if (!host && cudaMalloc(&rowsum, w.ny * sizeof(double)) != cudaSuccess) {
+    if (!host && swb::pool_malloc((void**)&rowsum, w.ny * sizeof(double)) != cudaSuccess) {
         (void)cudaGetLastError();
         return SW_ERR_NOMEM;
     }
     auto free_rowsum = [&] {
         if (host) std::free(rowsum);
-        else if (rowsum) cudaFree(rowsum);
+        else if (rowsum) {
+            cudaStreamSynchronize(A.s);
+            swb::pool_free(rowsum, w.ny * sizeof(double));
+        }
         rowsum = nullptr;
     };
     const bool segments = want_segments && A.stored;      // the segment's records fit
