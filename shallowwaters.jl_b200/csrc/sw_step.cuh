@@ -29,25 +29,64 @@
 // lanes beside the overlap write the 3 columns that the other half cannot
 // compute (it lacks their neighbours) into it.
 //
-// Measured (B200, per step without the tracer; four stage launches and the
-// tail before): 2048x1024 Float32 124 us against 160, 1000x500 43 against 90,
-// 512x256 Float64 28 against 57.  The 108 x 47 tile of 63 rows takes 57
-// thousand clocks: load 6, A 4 x 3.8, B 4 x 7.6, T1 5, T2 7.7.  B issues in
-// four tenths of its slots (sixteen warps of 128 registers, each row a chain
-// of loads and packed adds); variants of 20, 24 and 32 warps with fewer
-// registers took the same time at this size.  On small grids the passes'
-// latencies (about 1000 clocks each) and the launch are the time.
+// Order at the start.  What no earlier launch writes (a thread's columns and
+// ghost places, the rows' static fields) is formed before the wait for the
+// launch before, which it overlaps: 64x32 12.6 -> 10.8 us a step, 512x256
+// 23.8 -> 22.4.  The stop flag is read beside the state.
+//
+// Measured (B200, us per step with the tracer beside it; the four stage
+// launches and the tail before): 64x32 24.5 -> 10.7, 256x128 26.3 -> 11.8,
+// 512x256 49.9 -> 21.5, 1000x500 over a ridge 89 -> 38.5, 2048x1024 181 -> 125,
+// 512x256 Float64 60 -> 25.6, SSPRK3 500x250 42.4 -> 27.5.  The 103 x 47 tile
+// of 63 rows takes 65 thousand clocks: load 6, A 4 x 4.2, B 4 x 7.5, T1 5, T2
+// 7.5, the rest start and end.  A third of the issue slots are used (sixteen
+// warps of 128 registers); a warp waits most for the fixed latency of its
+// packed adds, then for barriers, loads and the shared memory about equally.
+// 20, 24 and 32 warps with fewer registers, passes A, T1 and T2 unrolled by 4
+// and a division on packs took as long or longer.  A tile of a small grid
+// takes 13 thousand clocks, 700 to 1100 a pass, which are the latencies of one
+// row, and the launch.
 #pragma once
 #include <type_traits>
 
 #include "sw_common.cuh"
 #include "sw_ghost.cuh"
 #include "sw_pack.cuh"
+#include "sw_storage.cuh"
 
 namespace swb {
 
 constexpr int STEP_LO = 10, STEP_HI = 6;   // halo below and above a tile: 4 RK stages and the tail
 constexpr int STEP_LO_SSP = 10, STEP_HI_SSP = 10;   // 4 SSP sub-stages and the tail
+
+// How a tile reads the state, forms a stage's results and writes the new
+// state.  StepNative: arrays of T.  Step16: the 16-bit storage form
+// (sw_s16.cuh): pairs hi + lo scaled by s; a stage's increment b*d is rounded
+// to 16 bits before it is added to the state, and so is the accumulated
+// increment, which then takes the place of the accumulator X0.
+struct StepNative {
+    static constexpr bool S16 = false;
+};
+template <class E>
+struct Step16 {
+    static constexpr bool S16 = true;
+    E* h[2][3];                         // hi of u, v, eta: the step's start, the new state
+    E* l[2][3];                         // lo
+    float s, inv_s;                     // scale and its inverse (powers of two)
+    __device__ __forceinline__ float get(int f, int o) const { return (from16(h[0][f][o]) + from16(l[0][f][o])) * inv_s; }
+    __device__ __forceinline__ void put(int f, int o, float x) const {
+        const float y = x * s;
+        const E hi = to16<E>(y);
+        h[1][f][o] = hi;
+        l[1][f][o] = to16<E>(y - from16(hi));
+    }
+    // the value that 16 bits keep of x
+    __device__ __forceinline__ float keep(float x) const { return from16(to16<E>(x * s)) * inv_s; }
+    __device__ __forceinline__ Pack<float>::P keep(Pack<float>::P x) const {
+        using K = Pack<float>;
+        return K::make(keep(K::get<0>(x)), keep(K::get<1>(x)));
+    }
+};
 
 // Sub-stage updates (src/time_integration.jl:80-196): axb!, the kn stage's
 // dxaybzc!, 4SSPRK3's caxb! and cxab!
@@ -112,8 +151,8 @@ struct StepShape {
 // PV_Sadourny! instead of PV_ArakawaHsu!.  EDGE is false for tiles none of
 // whose points is a ghost, a ghost source or a wall.  HVAR: the depth varies along x (an array in shared
 // memory; else one value per row).
-template <class T, class SH, bool HVAR, bool SSP, bool SAD, bool EDGE>
-__device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>::P* sm, int xs, int xe, int zx,
+template <class T, class SH, bool HVAR, bool SSP, bool SAD, bool EDGE, class IO>
+__device__ __forceinline__ void step_tile(const StepArgs<T>& A, const IO& io, typename Pack<T>::P* sm, int xs, int xe, int zx,
                                           int ys, int ye, int zy, int zy1, bool whole) {
     using K = Pack<T>;
     using P = typename K::P;
@@ -175,56 +214,30 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
     // EDGE only: what the thread's columns are
     bool cu[V];                                           // u interior
     bool zero = false;                                    // one of the columns is 0 of a periodic domain
-    bool wrap = false;                                    // one of the columns is -1 of a periodic domain
+    bool wc[V], wrap = false;                             // a column is -1 of a periodic domain
 #pragma unroll
     for (int h = 0; h < V; h++) {
         cu[h] = cv[h] && X[h] >= (per ? 0 : 1) && X[h] < N;
         zero = zero || (per && cv[h] && X[h] == 0);
-        wrap = wrap || (per && cv[h] && X[h] == -1);
+        wc[h] = EDGE && per && cv[h] && X[h] == -1;
+        wrap = wrap || wc[h];
     }
     P x0u[SSP ? 1 : R], x0v[SSP ? 1 : R], x0e[SSP ? 1 : R];   // RK: the accumulator X0 of this thread's points
+    // RK: the step's state of this thread's points, where there are registers for it (512x256, four rows: 23.7 us a
+    // step against 24.6 with a load per stage)
+    constexpr bool KEEPX = !SSP && R <= 4;
+    P Xku[KEEPX ? R : 1], Xkv[KEEPX ? R : 1], Xke[KEEPX ? R : 1];
     bool keep[V];                                         // nonperiodic u column that keeps its value
 #pragma unroll
     for (int h = 0; h < V; h++) keep[h] = EDGE && cv[h] && !per && X[h] >= -1 && (X[h] <= 0 || X[h] >= N);
+    bool ring[V];                                         // ... and is not an output column, but this tile's to write
+#pragma unroll
+    for (int h = 0; h < V; h++)
+        ring[h] = keep[h] && !own[h] && (X[h] == -1 || X[h] >= N) && (X[h] < 0 ? xs == 0 : xe == N) &&
+                  (V == 1 || (h == 0 ? lx <= EW - 3 : lx >= 2));
     // whether any lane's are
-    const bool wwrap = EDGE && __any_sync(0xffffffffu, wrap), wzero = EDGE && __any_sync(0xffffffffu, zero),
+    const bool wzero = EDGE && __any_sync(0xffffffffu, zero),
                wkeep = EDGE && __any_sync(0xffffffffu, !prod && (keep[0] || keep[V - 1]));
-
-    // ---- the step's state, halo and ghosts included
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-        const int ly = ly0 + i;
-        if (ly < EHv) {
-            T a[V], b[V], c[V], d[V];
-#pragma unroll
-            for (int h = 0; h < V; h++) {
-                a[h] = b[h] = c[h] = T(0);
-                d[h] = T(1);
-                if (!EDGE || cv[h]) {
-                    const int o = gofs(h, zy + ly);
-                    a[h] = A.uX[o]; b[h] = A.vX[o]; c[h] = A.eX[o];
-                    if (HVAR) {
-                        const T w = A.H.at(X[h], zy + ly);
-                        d[h] = (X[h] >= -1 && X[h] <= N) ? w : T(1);
-                    }
-                }
-            }
-            const int s = ly * EW + lx;
-            su[s] = K::make(a[0], a[V - 1]);
-            sv[s] = K::make(b[0], b[V - 1]);
-            se[s] = K::make(c[0], c[V - 1]);
-            if constexpr (!SSP) { x0u[i] = su[s]; x0v[i] = sv[s]; x0e[i] = se[s]; }
-            if (HVAR) sH[s] = K::make(d[0], d[V - 1]);
-        }
-    }
-    for (int ly = threadIdx.x; ly < EHv; ly += SH::NW * 32) {
-        const int y = zy + ly + ROW0;
-        if (!HVAR) tH[ly] = K::all(A.H.p[y * A.H.sy]);
-        tf[ly] = K::all(A.fq.p[y * A.fq.sy]);
-        tFx[ly] = K::all(A.Fxt * A.Fx.p[y * A.Fx.sy]);
-        tFy[ly] = K::all(A.Fyt * A.Fy.p[y * A.Fy.sy]);
-    }
-    __syncthreads();
 
     // stores the updated pack of index s.  Ghost points and columns outside the
     // domain receive values without meaning here: ghosts() fills the former,
@@ -243,46 +256,148 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
     };
     // EDGE: ghost points of u, v, eta (src/ghost_points.jl:46-133), spread over
     // the block: columns -2, -1, N, N+1 of every row, then rows -2, -1, M, M+1
-    // of every column.  Neither part reads what the other writes.
-    auto ghosts = [&]() {
-        auto from = [&](P* f, int rel, int ly) {
-            return V == 1 || rel < EW - 2 ? at(f, ly * EW + rel, 0) : at(f, ly * EW + rel - SHIFT, V - 1);
-        };
-        auto put = [&](P* f, int rel, int ly, T val) {
-            if (rel < EW) at(f, ly * EW + rel, 0) = val;
-            if (V == 2 && rel >= SHIFT) at(f, ly * EW + rel - SHIFT, V - 1) = val;
-        };
-        const T oma = A.gr.oma;
-        const bool seam = per && !whole;
-        for (int t = threadIdx.x; t < 4 * EH; t += SH::NW * 32) {
+    // of every column; at most one of each kind per thread.  Neither kind reads
+    // what the other writes.  Their places: a source, a place (with a mark
+    // if the other half holds that column too), eta's source.
+    constexpr int BOTH = 1 << 30;
+    auto place = [&](int rel, int ly) {
+        return rel < EW ? (ly * EW + rel) * V | (V == 2 && rel >= SHIFT ? BOTH : 0) : (ly * EW + rel - SHIFT) * V + V - 1;
+    };
+    auto source = [&](int rel, int ly) {
+        return V == 1 || rel < EW - 2 ? (ly * EW + rel) * V : (ly * EW + rel - SHIFT) * V + V - 1;
+    };
+    auto put = [&](P* f, int at_, T val) {
+        const int q = at_ & ~BOTH;
+        scalar(f)[q] = val;
+        if (at_ & BOTH) scalar(f)[q - SHIFT * V + V - 1] = val;
+    };
+    struct Places {
+        int c_src = -1, c_dst = 0, c_eta = -1, c_ofs = 0;     // a column's ghost; where it is in the fields' arrays
+        int r_src = -1, r_dst = 0, r_ofs = 0;                 // a row's ghost
+        bool r_u = false, r_e = false;
+        bool c_out = false, c_oute = false, r_outu = false, r_oute = false;   // ghosts of this tile's outputs
+    };
+    auto find = [&]() {
+        Places G;
+        static_assert(4 * EH <= SH::NW * 32 && 512 <= SH::NW * 32, "one ghost of each kind per thread");
+        const int t = threadIdx.x;
+        if (t < 4 * EH) {
             const int j = t & 3, ly = t >> 2, y = zy + ly;
-            // the j-th ghost column's place, its column and the distance to its source
+            const bool seam = per && !whole;
             const int gx = j < 2 ? j - 2 : N + j - 2;
             const int rel = (seam ? (j < 2 ? gx : gx - (N + 4)) + (zx < -2 ? 0 : N + 4) : gx) - zx;
             const int d = per ? (whole ? (j < 2 ? N : -N) : (j < 2 ? -4 : 4)) : (j == 0 ? 3 : j == 1 ? 1 : j == 2 ? -1 : -3);
             if (ly < EHv && rel >= 0 && rel < SH::COLS && rel + d >= 0 && rel + d < SH::COLS) {
-                if (per) put(su, rel, ly, from(su, rel + d, ly));
-                const T w = from(sv, rel + d, ly);
-                put(sv, rel, ly, per ? w : oma * w);
-                if (j == 1 || j == 2) {                   // eta: the corners take the column-copied value
-                    const int src = min(max(ly, -zy), M - 1 - zy);
-                    if (y >= -1 && y <= M) put(se, rel, ly, from(se, rel + d, src));
+                G.c_src = source(rel + d, ly);
+                G.c_dst = place(rel, ly);
+                G.c_ofs = (y + ROW0) * g.P + gx + COL0;
+                // eta: one ghost column each side; the corners take the column-copied value
+                if ((j == 1 || j == 2) && y >= -1 && y <= M) G.c_eta = source(rel + d, min(max(ly, -zy), M - 1 - zy));
+                const bool mine = rel + d >= xs - zx && rel + d < xe - zx;
+                G.c_out = mine && y >= (ys == 0 ? -1 - per : ys) && y < (ye == M ? M + 2 : ye);
+                G.c_oute = mine && y >= (ys == 0 ? -1 : ys) && y < (ye == M ? M + 1 : ye);
+            }
+        }
+        if ((lowwall || highwall) && t < 512) {
+            const int j = t >> 7, rel = t & 127;
+            const int y = j < 2 ? j - 2 : M + j - 2, ly = y - zy;
+            const int d = j == 0 ? 3 : j == 1 ? 1 : j == 2 ? -1 : -3;
+            int x = zx + rel;
+            if (per && x < -2) x += N + 4;
+            else if (per && !whole && x > N + 1) x -= N + 4;
+            if (rel < SH::COLS && ly >= 0 && ly < EHv && x >= -1 && x <= N + 1) {
+                G.r_u = !per;
+                G.r_e = (j == 1 || j == 2) && x >= 0 && x < N;
+                if (G.r_u || G.r_e) {
+                    G.r_src = source(rel, ly + d);
+                    G.r_dst = place(rel, ly);
+                    G.r_ofs = (y + ROW0) * g.P + x + COL0;
+                    const bool in = rel >= xs - zx && rel < xe - zx, wall = j < 2 ? ys == 0 : ye == M;
+                    G.r_outu = wall && (in || (x < 0 && xs == 0) || (x >= N && xe == N));
+                    G.r_oute = wall && in;
                 }
             }
         }
-        if (lowwall || highwall)
-            for (int t = threadIdx.x; t < 4 * 128; t += SH::NW * 32) {
-                const int j = t >> 7, rel = t & 127;
-                const int y = j < 2 ? j - 2 : M + j - 2, ly = y - zy;
-                const int d = j == 0 ? 3 : j == 1 ? 1 : j == 2 ? -1 : -3;
-                int x = zx + rel;
-                if (per && x < -2) x += N + 4;
-                else if (per && !whole && x > N + 1) x -= N + 4;
-                if (rel < SH::COLS && ly >= 0 && ly < EHv && x >= -1 && x <= N + 1) {
-                    if (!per) put(su, rel, ly, oma * from(su, rel, ly + d));
-                    if ((j == 1 || j == 2) && x >= 0 && x < N) put(se, rel, ly, from(se, rel, ly + d));
+        return G;
+    };
+    // What the stages need of them, in one register each (found anew in each stage they took 500 of a ghost pass's
+    // 900 clocks, kept as they are the registers of the four-row tiles and more): source, place and its mark, and what eta does (1 the same,
+    // 2 and 3 the row after or before: the corners) or which of u and eta there is.
+    static_assert(NP * V <= 8192, "13 bits for a place");
+    int col_ghost = -1, row_ghost = -1;
+    if (EDGE) {
+        const Places G = find();
+        const int eta = G.c_eta < 0 ? 0 : G.c_eta == G.c_src ? 1 : G.c_eta > G.c_src ? 2 : 3;
+        auto packed = [](int src, int dst, int how) {
+            return src < 0 ? -1 : src | (dst & ~BOTH) << 13 | (dst & BOTH ? 1 << 26 : 0) | how << 27;
+        };
+        col_ghost = packed(G.c_src, G.c_dst, eta);
+        row_ghost = packed(G.r_src, G.r_dst, G.r_u + 2 * G.r_e);
+    }
+
+    // the rows' static fields; up to here nothing depends on the launch before
+    // this one, which may still run
+    for (int ly = threadIdx.x; ly < EHv; ly += SH::NW * 32) {
+        const int y = zy + ly + ROW0;
+        if (!HVAR) tH[ly] = K::all(A.H.p[y * A.H.sy]);
+        tf[ly] = K::all(A.fq.p[y * A.fq.sy]);
+        tFx[ly] = K::all(A.Fxt * A.Fx.p[y * A.Fx.sy]);
+        tFy[ly] = K::all(A.Fyt * A.Fy.p[y * A.Fy.sy]);
+    }
+    cudaGridDependencySynchronize();
+    const int stop = A.st->stop;
+    // ---- the step's state, halo and ghosts included
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        const int ly = ly0 + i;
+        if (ly < EHv) {
+            T a[V], b[V], c[V], d[V];
+#pragma unroll
+            for (int h = 0; h < V; h++) {
+                a[h] = b[h] = c[h] = T(0);
+                d[h] = T(1);
+                if (!EDGE || cv[h]) {
+                    const int o = gofs(h, zy + ly);
+                    if constexpr (IO::S16) { a[h] = io.get(0, o); b[h] = io.get(1, o); c[h] = io.get(2, o); }
+                    else { a[h] = A.uX[o]; b[h] = A.vX[o]; c[h] = A.eX[o]; }
+                    if (HVAR) {
+                        const T w = A.H.at(X[h], zy + ly);
+                        d[h] = (X[h] >= -1 && X[h] <= N) ? w : T(1);
+                    }
                 }
             }
+            const int s = ly * EW + lx;
+            su[s] = K::make(a[0], a[V - 1]);
+            sv[s] = K::make(b[0], b[V - 1]);
+            se[s] = K::make(c[0], c[V - 1]);
+            if constexpr (IO::S16) x0u[i] = x0v[i] = x0e[i] = K::all(T(0));
+            else if constexpr (!SSP) { x0u[i] = su[s]; x0v[i] = sv[s]; x0e[i] = se[s]; }
+            if constexpr (KEEPX) { Xku[i] = su[s]; Xkv[i] = sv[s]; Xke[i] = se[s]; }
+            if (HVAR) sH[s] = K::make(d[0], d[V - 1]);
+        }
+    }
+    if (stop) return;                                     // read beside the state
+    __syncthreads();
+
+    const T oma = A.gr.oma;
+    auto ghosts = [&]() {
+        auto dst = [](int p) { return (p >> 13 & 8191) | (p >> 26 & 1 ? BOTH : 0); };
+        if (col_ghost >= 0) {
+            const int src = col_ghost & 8191, to = dst(col_ghost), eta = col_ghost >> 27;
+            if (per) put(su, to, scalar(su)[src]);
+            const T w = scalar(sv)[src];
+            put(sv, to, per ? w : oma * w);
+            if (eta) put(se, to, scalar(se)[src + (eta == 2 ? EW * V : eta == 3 ? -EW * V : 0)]);
+        }
+        if (row_ghost >= 0) {
+            const int src = row_ghost & 8191, to = dst(row_ghost), how = row_ghost >> 27;
+            if (how & 1) put(su, to, oma * scalar(su)[src]);
+            if (how & 2) put(se, to, scalar(se)[src]);
+        }
+    };
+    auto out = [&](int f, int o, T val) {                 // a value of the new state
+        if constexpr (IO::S16) io.put(f, o, val);
+        else (f == 0 ? A.uo : f == 1 ? A.vo : A.eo)[o] = val;
     };
 
     const int stages = A.stages;
@@ -312,24 +427,13 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
                     const P hlh = K::add(hl, h);
                     const P hs = K::mul(q4, hlh, nz);
                     // PV! (src/PV_advection.jl:2-18)
-                    P q = K::div(K::sub(K::add(tf[ly], K::sub(v_c, v_l)), K::sub(u_c, u_m)), K::add(hs_m, hs));
-                    if (EDGE && wwrap) {
-                        // column -1 evaluates q[end] (src/PV_advection.jl:110,126) at column N, with its own Coriolis value
-#pragma unroll
-                        for (int hh = 0; hh < V; hh++)
-                            if (cv[hh] && X[hh] == -1) {
-                                int rel = lx + hh * SHIFT + (whole ? N + 1 : -3), ha = 0;
-                                if (V == 2 && rel >= EW) { rel -= SHIFT; ha = V - 1; }
-                                const int w = ly * EW + rel;
-                                auto hv = [&](int o, int row) { return at(se, o, ha) + (HVAR ? at(sH, o, ha) : at(tH, row, 0)); };
-                                const T qt = T(0.25);
-                                const T hq = qt * (hv(w - EW - 1, ly - 1) + hv(w - EW, ly - 1)) + qt * (hv(w - 1, ly) + hv(w, ly));
-                                const T qw = (at(tf, ly, 0) + (at(sv, w, ha) - at(sv, w - 1, ha)) -
-                                              (at(su, w, ha) - at(su, w - EW, ha))) / hq;
-                                q = K::pick(K::all(qw), q, hh == 0, hh == 1);
-                            }
+                    const P q = K::div(K::sub(K::add(tf[ly], K::sub(v_c, v_l)), K::sub(u_c, u_m)), K::add(hs_m, hs));
+                    if (EDGE && wrap) {                     // but column -1: see below
+                        if (!wc[0]) at(sq, s, 0) = K::template get<0>(q);
+                        if (V == 2 && !wc[V - 1]) at(sq, s, V - 1) = K::template get<V - 1>(q);
+                    } else {
+                        sq[s] = q;
                     }
-                    sq[s] = q;
                     sU[s] = K::mulx(u_c, K::mulx(half, hlh));           // Uflux!/Vflux! (src/rhs.jl:277-304)
                     sV[s] = K::mulx(v_c, K::mulx(half, K::add(h, h_m)));
                     // bernoulli! (src/rhs.jl:162-180)
@@ -341,12 +445,47 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
                 }
             }
         }
+        if (EDGE && per) {
+            // Column -1 evaluates q[end] (src/PV_advection.jl:110,126) at column N, with its own Coriolis value: a thread
+            // per row (its lane held up its warp in every row: pass A of such a tile 6.2 thousand clocks instead of 4.2).
+            const int rel = -1 - zx + (whole || zx < -2 ? 0 : N + 4), ly = threadIdx.x;
+            if (rel >= 0 && rel < SH::COLS && ly >= a0 && ly < a1) {
+                int w = rel + (whole ? N + 1 : -3), ha = 0;
+                if (V == 2 && w >= EW) { w -= SHIFT; ha = V - 1; }
+                w += ly * EW;
+                auto hv = [&](int o, int row) { return at(se, o, ha) + (HVAR ? at(sH, o, ha) : at(tH, row, 0)); };
+                const T qt = T(0.25);
+                const T hq = qt * (hv(w - EW - 1, ly - 1) + hv(w - EW, ly - 1)) + qt * (hv(w - 1, ly) + hv(w, ly));
+                put(sq, place(rel, ly), (at(tf, ly, 0) + (at(sv, w, ha) - at(sv, w - 1, ha)) -
+                                         (at(su, w, ha) - at(su, w - EW, ha))) / hq);
+            }
+        }
+        // X, for the next stage's input or the kn stage's snapshot, one row ahead (RK: not used on the last stage, and
+        // the first row before the barrier, whose wait then hides the load: 2048x1024 134.5 -> 131.2 us a step; SSP
+        // 29.2 -> 29.6, so not there)
+        int o = gofs(0, zy + ly0);
+        const int dX = EDGE ? X[V - 1] - X[0] : (V - 1) * SHIFT;
+        P Xu = K::all(T(0)), Xv = Xu, Xe = Xu;
+        auto loadX = [&]() {
+            if constexpr (IO::S16) {
+                Xu = K::make(io.get(0, o), io.get(0, o + dX));
+                Xv = K::make(io.get(1, o), io.get(1, o + dX));
+                Xe = K::make(io.get(2, o), io.get(2, o + dX));
+            } else {
+                Xu = K::make(A.uX[o], A.uX[o + dX]);
+                Xv = K::make(A.vX[o], A.vX[o + dX]);
+                Xe = K::make(A.eX[o], A.eX[o + dX]);
+            }
+            o += g.P;
+        };
+        if (!SSP && !KEEPX && ly0 < EHv) loadX();
         __syncthreads();
         // ---- pass B: tendencies and the stage combination, in place (SUB: enum StepSub, -1 for RK)
         auto pass_b = [&](auto subc) {
             constexpr int SUB = decltype(subc)::value;
             const int b0 = lowwall ? 0 : ay + 2, b1 = highwall ? EHv : by - 1;
-            const P a = A.a[k], b = A.b[k], o12 = A.o12;
+            [[maybe_unused]] const P a = A.a[k], b = A.b[k];
+            const P o12 = A.o12;
             [[maybe_unused]] const P x = A.x[k], kna = A.kna, knb = A.knb;
             if (ly0 < b1 && ly0 + R > b0) {
                 int s = ly0 * EW + lx;
@@ -362,22 +501,13 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
                     const P qbr = K::mulx(o12, K::add(K::add(qmr, q_r), q_c));
                     qhu_part = K::add(K::mul(qa, sU[s - EW], nz), K::mul(qbr, sU[s - EW + 1], nz));
                 }
-                // X, for the next stage's input or the kn stage's snapshot, one row ahead (RK: not used on the last stage)
-                int o = gofs(0, zy + ly0);
-                const int dX = EDGE ? X[V - 1] - X[0] : (V - 1) * SHIFT;
-                P Xu, Xv, Xe;
-                auto loadX = [&]() {
-                    Xu = K::make(A.uX[o], A.uX[o + dX]);
-                    Xv = K::make(A.vX[o], A.vX[o + dX]);
-                    Xe = K::make(A.eX[o], A.eX[o + dX]);
-                    o += g.P;
-                };
-                constexpr bool needX = SUB == -1 || SUB == STEP_KN;
-                if (needX) loadX();
+                constexpr bool needX = !KEEPX && (SUB == -1 || SUB == STEP_KN);
+                if (SSP && needX) loadX();
 #pragma unroll (SSP ? (R < 4 ? R : 4) : R)
                 for (int i = 0; i < R; i++) {
                     const int ly = ly0 + i, y = zy + ly;
-                    const P Xu_ = Xu, Xv_ = Xv, Xe_ = Xe;
+                    const P Xu_ = KEEPX ? Xku[KEEPX ? i : 0] : Xu, Xv_ = KEEPX ? Xkv[KEEPX ? i : 0] : Xv;
+                    [[maybe_unused]] const P Xe_ = KEEPX ? Xke[KEEPX ? i : 0] : Xe;
                     if (needX && i + 1 < R) loadX();
                     const P qn_c = sq[s + EW], qn_l = sq[s + EW - 1], qn_r = sq[s + EW + 1];
                     const P Vn_c = sV[s + EW], Vn_l = sV[s + EW - 1];
@@ -429,13 +559,22 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
                         store_u(s, update(su[s], Xu_, du));
                         store(sv, s, update(sv[s], Xv_, dv));
                     } else {
-                        x0u[i] = K::add(x0u[i], K::mul(a, du, nz));                 // axb!
-                        x0v[i] = K::add(x0v[i], K::mul(a, dv, nz));
-                        x0e[i] = K::sub(x0e[i], K::mul(a, ds, nz));
-                        P nu = K::add(Xu_, K::mul(b, du, nz));                       // caxb!
-                        P nv = K::add(Xv_, K::mul(b, dv, nz));
-                        P ne = K::sub(Xe_, K::mul(b, ds, nz));
-                        if (last) { nu = x0u[i]; nv = x0v[i]; ne = x0e[i]; }
+                        const P Du = K::add(x0u[i], K::mul(a, du, nz));             // axb!
+                        const P Dv = K::add(x0v[i], K::mul(a, dv, nz));
+                        const P De = K::sub(x0e[i], K::mul(a, ds, nz));
+                        P bu = K::mul(b, du, nz), bv = K::mul(b, dv, nz), be = K::mul(b, ds, nz);
+                        if constexpr (IO::S16) {
+                            bu = io.keep(bu); bv = io.keep(bv); be = io.keep(be);
+                            x0u[i] = io.keep(Du); x0v[i] = io.keep(Dv); x0e[i] = io.keep(De);
+                        } else {
+                            x0u[i] = Du; x0v[i] = Dv; x0e[i] = De;
+                        }
+                        P nu = K::add(Xu_, bu), nv = K::add(Xv_, bv), ne = K::sub(Xe_, be);      // caxb!
+                        if (last) {
+                            nu = IO::S16 ? K::add(Xu_, Du) : Du;
+                            nv = IO::S16 ? K::add(Xv_, Dv) : Dv;
+                            ne = IO::S16 ? K::add(Xe_, De) : De;
+                        }
                         store_u(s, nu);
                         store(sv, s, nv);
                         store(se, s, ne);
@@ -561,16 +700,21 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
             const P cD = A.cD, rD = A.rD, Dt = A.Dt_diff, nuB = A.nuB;
             int s = r0 * EW + lx;
             P nq_c = nuB, nq_r = nuB, S12_c = nuB, S22_m = nuB, sK_m = nuB, h_m = nuB;
+            P n_l = nuB, n_c = nuB, n_r = nuB, Lu_c = nuB, Lv_c = nuB;
             if (A.tail) {
                 P n_m = nuB;
+                Lu_c = sU[s];
+                Lv_c = sV[s];
                 if (smag) {
                     n_m = sq[s - EW];
-                    const P nl = sq[s - 1], nc = sq[s], nr = sq[s + 1];
-                    nq_c = K::add(K::mul(q4, K::add(sq[s - EW - 1], n_m), nz), K::mul(q4, K::add(nl, nc), nz));
-                    nq_r = K::add(K::mul(q4, K::add(n_m, sq[s - EW + 1]), nz), K::mul(q4, K::add(nc, nr), nz));
+                    n_l = sq[s - 1];
+                    n_c = sq[s];
+                    n_r = sq[s + 1];
+                    nq_c = K::add(K::mul(q4, K::add(sq[s - EW - 1], n_m), nz), K::mul(q4, K::add(n_l, n_c), nz));
+                    nq_r = K::add(K::mul(q4, K::add(n_m, sq[s - EW + 1]), nz), K::mul(q4, K::add(n_c, n_r), nz));
                 }
-                S22_m = K::mul(n_m, K::sub(sV[s], sV[s - EW]), nz);
-                S12_c = K::mul(nq_c, K::sub(sU[s], sU[s - EW]), nz);
+                S22_m = K::mul(n_m, K::sub(Lv_c, sV[s - EW]), nz);
+                S12_c = K::mul(nq_c, K::sub(Lu_c, sU[s - EW]), nz);
                 if (quad) {
                     sK_m = sp[s - EW];
                     h_m = K::add(se[s - EW], HVAR ? sH[s - EW] : tH[max(r0 - 1, 0)]);
@@ -582,13 +726,11 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
                 const P u_c = su[s], v_c = sv[s];
                 P nu = u_c, nv = v_c;
                 if (A.tail) {
-                    const P Lu_l = sU[s - 1], Lu_c = sU[s], Lu_r = sU[s + 1], Lu_n = sU[s + EW];
-                    const P Lv_l = sV[s - 1], Lv_c = sV[s], Lv_r = sV[s + 1], Lv_n = sV[s + EW];
-                    P n_l = nuB, n_c = nuB, nqn_c = nuB, nqn_r = nuB;
+                    const P Lu_l = sU[s - 1], Lu_r = sU[s + 1], Lu_n = sU[s + EW];
+                    const P Lv_l = sV[s - 1], Lv_r = sV[s + 1], Lv_n = sV[s + EW];
+                    P nnl = nuB, nnc = nuB, nnr = nuB, nqn_c = nuB, nqn_r = nuB;
                     if (smag) {
-                        n_l = sq[s - 1]; n_c = sq[s];
-                        const P n_r = sq[s + 1];
-                        const P nnl = sq[s + EW - 1], nnc = sq[s + EW], nnr = sq[s + EW + 1];
+                        nnl = sq[s + EW - 1]; nnc = sq[s + EW]; nnr = sq[s + EW + 1];
                         nqn_c = K::add(K::mul(q4, K::add(n_l, n_c), nz), K::mul(q4, K::add(nnl, nnc), nz));
                         nqn_r = K::add(K::mul(q4, K::add(n_c, n_r), nz), K::mul(q4, K::add(nnc, nnr), nz));
                     }
@@ -615,80 +757,90 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, typename Pack<T>
                     nu = K::add(u_c, K::mul(Dt, K::add(K::add(Bu, LLu1), LLu2), nz));
                     nv = K::add(v_c, K::mul(Dt, K::add(K::add(Bv, LLv1), LLv2), nz));
                     S12_c = S12_n; S22_m = S22; nq_c = nqn_c; nq_r = nqn_r;
+                    n_l = nnl; n_c = nnc; n_r = nnr; Lu_c = Lu_n; Lv_c = Lv_n;
                 }
+                const P ne = se[s];
                 if (!EDGE) {
-                    const P ne = se[s];
                     const int o = gofs(0, y);
                     if (own[0]) {
-                        A.uo[o] = K::template get<0>(nu);
-                        A.vo[o] = K::template get<0>(nv);
-                        A.eo[o] = K::template get<0>(ne);
+                        out(0, o, K::template get<0>(nu));
+                        out(1, o, K::template get<0>(nv));
+                        out(2, o, K::template get<0>(ne));
                     }
                     if (V == 2 && own[V - 1]) {
-                        A.uo[o + SHIFT] = K::template get<V - 1>(nu);
-                        A.vo[o + SHIFT] = K::template get<V - 1>(nv);
-                        A.eo[o + SHIFT] = K::template get<V - 1>(ne);
+                        out(0, o + SHIFT, K::template get<V - 1>(nu));
+                        out(1, o + SHIFT, K::template get<V - 1>(nv));
+                        out(2, o + SHIFT, K::template get<V - 1>(ne));
                     }
                 } else {
-                    // into shared memory, for the ghost points; untouched halo cells keep their value
+                    // untouched halo cells keep their value; the nonperiodic u columns among them belong to the
+                    // first and the last tile
                     const bool row = y >= 0 && y < M;
-                    su[s] = K::pick(nu, u_c, cu[0] && row, cu[V - 1] && row);
-                    if (row && y >= 1) sv[s] = nv;
+                    nu = K::pick(nu, u_c, cu[0] && row, cu[V - 1] && row);
+                    if (!row || y == 0) nv = v_c;
+                    su[s] = nu;                            // sources of the ghost points
+                    sv[s] = nv;
+#pragma unroll
+                    for (int h = 0; h < V; h++) {
+                        const int o = gofs(h, y);
+                        if (per ? own[h] : row && (own[h] || ring[h])) out(0, o, h ? K::template get<V - 1>(nu) : K::template get<0>(nu));
+                        if (own[h] && y != -2) out(1, o, h ? K::template get<V - 1>(nv) : K::template get<0>(nv));
+                        if (own[h] && row) out(2, o, h ? K::template get<V - 1>(ne) : K::template get<0>(ne));
+                    }
                 }
                 s += EW;
             }
         }
     }
     if (EDGE) {
+        // the outputs' ghost points
+        const Places G = find();
         __syncthreads();
-        ghosts();
-        __syncthreads();
-        // the tile's outputs, the untouched columns beside them (nonperiodic u) and the ghosts copied from them
-        const int t0 = ys == 0 ? -2 : ys, t1 = ye == M ? M + 2 : ye;
-        for (int h = 0; h < V; h++) {
-            const int rel = lx + h * SHIFT;
-            bool wr = rel >= xs - zx && rel < xe - zx;
-            if (X[h] < 0 || X[h] >= N) {
-                if (per) {
-                    const int src = rel + (X[h] < 0 ? (whole ? N : -4) : (whole ? -N : 4));
-                    wr = src >= xs - zx && src < xe - zx;
-                } else {
-                    wr = X[h] < 0 ? xs == 0 : xe == N;
-                }
-            }
-            wr = wr && cv[h] && (V == 1 || (h == 0 ? lx <= EW - 3 : lx >= 2));
-            if (!wr) continue;
-            for (int y = max(zy + ly0, t0); y < min(zy + ly0 + R, t1); y++) {
-                const int s = (y - zy) * EW + lx, o = gofs(h, y);
-                if (per || X[h] >= -1) A.uo[o] = at(su, s, h);
-                if (y >= -1) A.vo[o] = at(sv, s, h);
-                if (X[h] >= -1 && X[h] <= N && y >= -1 && y <= M) A.eo[o] = at(se, s, h);
-            }
+        if (G.c_out) {
+            if (per) out(0, G.c_ofs, scalar(su)[G.c_src]);
+            const T w = scalar(sv)[G.c_src];
+            if (zy + (int)(threadIdx.x >> 2) >= -1) out(1, G.c_ofs, per ? w : oma * w);
         }
+        if (G.c_oute && G.c_eta >= 0) out(2, G.c_ofs, scalar(se)[G.c_eta]);
+        if (G.r_outu && G.r_u) out(0, G.r_ofs, oma * scalar(su)[G.r_src]);
+        if (G.r_oute && G.r_e) out(2, G.r_ofs, scalar(se)[G.r_src]);
     }
 }
 
 // tile `tile` of the domain, by the calling block
-template <class T, class SH, bool HVAR, bool SSP, bool SAD>
-__device__ __forceinline__ void step_block(const StepArgs<T>& A, int tile, typename SH::P* sm) {
+template <class T, class SH, bool HVAR, bool SSP, bool SAD, class IO = StepNative>
+__device__ __forceinline__ void step_block(const StepArgs<T>& A, int tile, typename SH::P* sm, const IO& io = IO()) {
     const Geom& g = A.g;
     const bool whole = A.ntx == 1 && g.N + 4 <= SH::COLS;
     int xs, xe, zx, ys, ye, zy, zy1;
-    step_cols(g.N, g.ep, A.ntx, whole, A.lo, tile % A.ntx, xs, xe, zx);
-    step_rows(g.M, A.nty, A.lo, A.hi, tile / A.ntx, ys, ye, zy, zy1);
+    // tiles at the edges first: they take longer (a fifth), and would hold up the end of the last wave
+    int i = tile % A.ntx, j = tile / A.ntx;
+    if (A.ntx > 2 && A.nty > 2) {
+        const int ends = 2 * A.ntx, sides = 2 * (A.nty - 2);
+        if (tile < ends) {
+            j = tile < A.ntx ? 0 : A.nty - 1;
+        } else if (tile < ends + sides) {
+            i = (tile - ends) & 1 ? A.ntx - 1 : 0;
+            j = 1 + (tile - ends) / 2;
+        } else {
+            const int t = tile - ends - sides;
+            i = 1 + t % (A.ntx - 2);
+            j = 1 + t / (A.ntx - 2);
+        }
+    }
+    step_cols(g.N, g.ep, A.ntx, whole, A.lo, i, xs, xe, zx);
+    step_rows(g.M, A.nty, A.lo, A.hi, j, ys, ye, zy, zy1);
     const bool edge = zx < 2 || zx + SH::COLS > g.N - 2 || zy < 2 || zy1 > g.M - 2;
-    if (edge) step_tile<T, SH, HVAR, SSP, SAD, true>(A, sm, xs, xe, zx, ys, ye, zy, zy1, whole);
-    else step_tile<T, SH, HVAR, SSP, SAD, false>(A, sm, xs, xe, zx, ys, ye, zy, zy1, false);
+    if (edge) step_tile<T, SH, HVAR, SSP, SAD, true>(A, io, sm, xs, xe, zx, ys, ye, zy, zy1, whole);
+    else step_tile<T, SH, HVAR, SSP, SAD, false>(A, io, sm, xs, xe, zx, ys, ye, zy, zy1, false);
 }
 
 template <class T, class SH, bool HVAR, bool SSP, bool SAD>
 __global__ void __launch_bounds__(SH::NW * 32, 1) rk_step_kernel(const __grid_constant__ StepArgs<T> A) {
     extern __shared__ __align__(16) unsigned char step_smem[];
     // all blocks of this launch run at once on a small grid: the next launch may then be prepared
-    // beside it; nothing of the step before is read until it has ended
+    // beside it (step_tile waits for this one's end before it reads the state)
     cudaTriggerProgrammaticLaunchCompletion();
-    cudaGridDependencySynchronize();
-    if (A.st->stop) return;
     step_block<T, SH, HVAR, SSP, SAD>(A, (int)blockIdx.x, reinterpret_cast<typename SH::P*>(step_smem));
 }
 

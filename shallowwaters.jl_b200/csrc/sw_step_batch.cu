@@ -22,7 +22,6 @@ __global__ void __launch_bounds__(SH::NW * 32, 1) rk_step_batch(const __grid_con
     }
     if (*B.istep > B.nt[lo]) return;
     const StepArgs<float>& A = B.m[lo];
-    if (A.st->stop) return;
     step_block<float, SH, true, false, false>(A, (int)blockIdx.x - B.block0[lo],
                                               reinterpret_cast<typename SH::P*>(step_smem));
 }
@@ -89,7 +88,8 @@ cudaError_t step_batch_launch(int shape, StepBatch& b, cudaStream_t stream) {
     if (shape == 0) return go_batch<SS::S0>(b, nb, stream);
     if (shape == 1) return go_batch<SS::S1>(b, nb, stream);
     if (shape == 2) return go_batch<SS::S2>(b, nb, stream);
-    return go_batch<SS::S3>(b, nb, stream);
+    if (shape == 3) return go_batch<SS::S3>(b, nb, stream);
+    return go_batch<SS::S4>(b, nb, stream);
 }
 
 }  // namespace swb

@@ -11,26 +11,34 @@
 namespace swb {
 namespace {
 
-// Tile shapes (StepShape: warps side by side, warps, rows per thread, rows).
-// Shape 2 fills the shared memory of an SM; with a depth that varies along x
-// the eighth array costs it rows.
+// Tile shapes (StepShape: warps side by side, warps, rows per thread).  Low
+// tiles for grids that leave SMs idle: a pass is then one row's latency, and
+// more rows per block cost more clocks than their halos (64x32: 20 rows 10.7 us
+// a step, 24 11.2, 32 12.3; 256x128 needs 24 rows to run in one wave, 11.8
+// against 19.8).  32 rows fill the gap up to 512x256 (400x200: 14.7, else
+// 19.0), 2 warps side by side the ones above (512x256: 21.5 against 23.4).
+// The last shape fills the shared memory of an SM, for several waves
+// (2048x1024: 125 against 171); with a depth that varies along x the eighth
+// array costs it rows.
 template <class T, bool HVAR>
 struct Shapes;
 template <bool HVAR>
 struct Shapes<float, HVAR> {
     using S0 = StepShape<float, 1, 20, 1>;
     using S1 = StepShape<float, 1, 24, 1>;
-    using S2 = StepShape<float, 2, 16, 4>;
-    using S3 = StepShape<float, 2, 16, HVAR ? 7 : 8>;
+    using S2 = StepShape<float, 1, 16, 2>;
+    using S3 = StepShape<float, 2, 16, 4>;
+    using S4 = StepShape<float, 2, 16, HVAR ? 7 : 8>;
 };
 template <bool HVAR>
 struct Shapes<double, HVAR> {
     using S0 = StepShape<double, 1, 20, 1>;
-    using S1 = StepShape<double, 1, 16, 2>;
-    using S2 = StepShape<double, 1, 16, 4>;
-    using S3 = StepShape<double, 2, 16, 7>;
+    using S1 = StepShape<double, 1, 24, 1>;
+    using S2 = StepShape<double, 1, 16, 2>;
+    using S3 = StepShape<double, 1, 16, 4>;
+    using S4 = StepShape<double, 2, 16, 7>;
 };
-constexpr int NSHAPES = 4;
+constexpr int NSHAPES = 5;
 
 // Tiles in x of shapes with cols columns; 0 if the grid has no split.
 inline int split_cols(int N, int ep, int cols, int lo, int hi) {
@@ -49,7 +57,7 @@ std::array<ShapeInfo, NSHAPES> shape_infos() {
         using S = decltype(s);
         return ShapeInfo{S::COLS, S::EWW, S::EH};
     };
-    return {of(typename SS::S0{}), of(typename SS::S1{}), of(typename SS::S2{}), of(typename SS::S3{})};
+    return {of(typename SS::S0{}), of(typename SS::S1{}), of(typename SS::S2{}), of(typename SS::S3{}), of(typename SS::S4{})};
 }
 // a tile's clocks: its passes' latencies and barriers, and its rows, measured
 inline double tile_clocks(const ShapeInfo& f, int rows) { return 7000.0 + 540.0 * f.EWW * rows; }
@@ -83,16 +91,11 @@ StepPlan plan_of(const Geom& g, int nsm, int lo, int hi) {
     return best;
 }
 
-template <class T, class S, bool HVAR, bool SSP, bool SAD>
-cudaError_t go(const StepArgs<T>& a, cudaStream_t stream) {
-    auto kern = rk_step_kernel<T, S, HVAR, SSP, SAD>;
-    constexpr int smem = S::smem(HVAR);
-    static_assert(smem <= 227 * 1024, "tile beyond the shared memory of an SM");
-    static const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    // the launch is prepared while the kernel before it runs; the kernel waits for that one's end
+// a launch that is prepared while the kernel before it runs; the kernel waits for that one's end
+template <class S, class Kernel, class... Args>
+cudaError_t go_prepared(Kernel kern, int smem, int nblocks, cudaStream_t stream, const Args&... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = a.ntx * a.nty;
+    cfg.gridDim = nblocks;
     cfg.blockDim = S::NW * 32;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -101,7 +104,16 @@ cudaError_t go(const StepArgs<T>& a, cudaStream_t stream) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, a);
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <class T, class S, bool HVAR, bool SSP, bool SAD>
+cudaError_t go(const StepArgs<T>& a, cudaStream_t stream) {
+    auto kern = rk_step_kernel<T, S, HVAR, SSP, SAD>;
+    constexpr int smem = S::smem(HVAR);
+    static_assert(smem <= 227 * 1024, "tile beyond the shared memory of an SM");
+    static const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e != cudaSuccess ? e : go_prepared<S>(kern, smem, a.ntx * a.nty, stream, a);
 }
 
 template <class T, bool HVAR, bool SSP, bool SAD>
@@ -110,7 +122,8 @@ cudaError_t go_shape(int shape, const StepArgs<T>& a, cudaStream_t stream) {
     if (shape == 0) return go<T, typename SS::S0, HVAR, SSP, SAD>(a, stream);
     if (shape == 1) return go<T, typename SS::S1, HVAR, SSP, SAD>(a, stream);
     if (shape == 2) return go<T, typename SS::S2, HVAR, SSP, SAD>(a, stream);
-    return go<T, typename SS::S3, HVAR, SSP, SAD>(a, stream);
+    if (shape == 3) return go<T, typename SS::S3, HVAR, SSP, SAD>(a, stream);
+    return go<T, typename SS::S4, HVAR, SSP, SAD>(a, stream);
 }
 
 }  // namespace

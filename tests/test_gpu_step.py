@@ -52,7 +52,7 @@ def run(S, Prog, n):
 
 # columns and rows around the tile widths (60, 124 and 32, 64 local columns; tiles hold 16 fewer, 20 at a seam) and
 # heights (32, 56 and 64 rows), and the smallest grids
-@pytest.mark.parametrize("shape", ["0", "1", "2", "3"])
+@pytest.mark.parametrize("shape", ["0", "1", "2", "3", "4"])
 @pytest.mark.parametrize("size", [(4, 1), (28, 1), (56, 1), (57, 1), (61, 3), (121, 2), (125, 5)])
 def test_tile_shapes_against_the_oracle(size, shape, monkeypatch):
     monkeypatch.setenv("SWB200_STEP", shape)
@@ -67,7 +67,7 @@ def test_tile_shapes_against_the_oracle(size, shape, monkeypatch):
 
 
 @pytest.mark.parametrize("rows", ["2", "5", "15", "16", "38", "47"])
-@pytest.mark.parametrize("shape", ["0", "1", "2", "3"])
+@pytest.mark.parametrize("shape", ["0", "1", "2", "3", "4"])
 def test_tile_heights_against_the_launches_per_stage(shape, rows, monkeypatch):
     for kw in OPTIONS[:6]:
         S, Prog = setup(dict(kw, nx=211, L_ratio=2))
