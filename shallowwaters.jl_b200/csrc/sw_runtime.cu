@@ -492,13 +492,18 @@ struct Engine : EngineBase {
                !c.surface_forcing && fmt_size(c.Tcomm) >= sizeof(T) && ctx->fq.sx == 0 && ctx->Fx.sx == 0 &&
                ctx->Fy.sx == 0;
     }
+    // Whether a context may take whole-step launches at all.  Settings of the
+    // launches per stage make those run.  Below 1024 cells a step keeps a launch
+    // per pass, as callers that count launches there expect (four stages, tail
+    // and tracer); SWB200_STEP overrides.
+    static bool step_launches(const sw_ctx* ctx) {
+        for (const char* k : {"SWB200_TMA", "SWB200_STAGE_BLOCKS", "SWB200_STAGE_TY", "SWB200_TAIL_TY"})
+            if (getenv(k)) return false;
+        return (long long)ctx->g.N * ctx->g.M >= 1024 || getenv("SWB200_STEP");
+    }
     int init(sw_ctx* ctx) {
         const sw_config& c = ctx->cfg;
-        for (const char* k : {"SWB200_TMA", "SWB200_STAGE_BLOCKS", "SWB200_STAGE_TY", "SWB200_TAIL_TY"})
-            if (getenv(k)) return SW_OK;             // settings of the launches per stage: these then run
-        // Below 1024 cells a step keeps a launch per pass, as callers that count launches there
-        // expect (four stages, tail and tracer); SWB200_STEP overrides.
-        if ((long long)ctx->g.N * ctx->g.M < 1024 && !getenv("SWB200_STEP")) return SW_OK;
+        if (!step_launches(ctx)) return SW_OK;
         if constexpr (STEP_TYPES)
             if (step_fits(ctx)) ctx->step_plan = step_plan<T>(ctx->g, ctx->nsm, ctx->H.sx != 0, c.time_scheme != SW_RK);
         return SW_OK;
@@ -1162,6 +1167,11 @@ struct Engine16 : Engine<float, float> {
                 if (int rc = alloc(p)) return rc;
         for (S16** p : {&sst16[0], &sst16[1]})
             if (int rc = alloc(p)) return rc;
+        // The whole-step kernel, where a ghost point's rounded increment is its source's (copies
+        // and (1-α) = ±1: a rounded multiple is not the multiple of the rounded otherwise).
+        if (this->step_launches(ctx) && this->step_fits(ctx) &&
+            (c.periodic || c.one_minus_alpha == 1.0 || c.one_minus_alpha == -1.0))
+            ctx->step_plan = step_plan<float>(ctx->g, ctx->nsm, ctx->H.sx != 0, false);
         return SW_OK;
     }
 
@@ -1298,41 +1308,57 @@ struct Engine16 : Engine<float, float> {
         const float Fxt = c.seasonal_wind_x ? (float)std::sin(c.omegaFx * (double)ctx->t) : 1.f;
         const float Fyt = c.seasonal_wind_y ? (float)std::sin(c.omegaFy * (double)ctx->t) : 1.f;
 
-        for (int k = 1; k <= c.RKo; k++) {
-            const S16StageArgs<S16> a = stage16_args(ctx, k, p, Fxt, Fyt);
-            const int nblk = (a.nsx * a.nsy + 3) / 4 + a.nring_blocks;
-            const bool first = k == 1, last = k == c.RKo;
-            const int rc = launch(ctx, 0, [&] {
-                if (g.ep) {
-                    if (first) stage16_ty<true, true, false>(a, nblk, ctx->stream, ctx->stage_ty);
-                    else if (last) stage16_ty<true, false, true>(a, nblk, ctx->stream, ctx->stage_ty);
-                    else stage16_ty<true, false, false>(a, nblk, ctx->stream, ctx->stage_ty);
-                } else {
-                    if (first) stage16_ty<false, true, false>(a, nblk, ctx->stream, ctx->stage_ty);
-                    else if (last) stage16_ty<false, false, true>(a, nblk, ctx->stream, ctx->stage_ty);
-                    else stage16_ty<false, false, false>(a, nblk, ctx->stream, ctx->stage_ty);
-                }
-            });
+        if (ctx->step_plan.shape >= 0) {
+            // stages and tail in one launch (sw_step.cuh)
+            const StepArgs<float> a = this->step_args(ctx, p, tail_now, Fxt, Fyt);
+            Step16<S16> io;
+            for (int k = 0; k < 2; k++) {
+                const F3 &h = hi[k ? q : p], &l = lo[k ? q : p];
+                io.h[k][0] = h.u; io.h[k][1] = h.v; io.h[k][2] = h.e;
+                io.l[k][0] = l.u; io.l[k][1] = l.v; io.l[k][2] = l.e;
+            }
+            io.s = s; io.inv_s = inv_s;
+            cudaError_t e = cudaSuccess;
+            const int rc = launch(ctx, 0, [&] { e = step16_launch(ctx->step_plan, a, io, ctx->H.sx != 0, ctx->stream); });
             if (rc) return rc;
-        }
-
-        if (tail_now) {
-            const TailArgs<float, float> t = tail16_args(ctx, p);
-            const TailStorePair<S16> o = tail16_out(p);
-            const int nb = (t.nsx * t.nsy + 3) / 4 + t.nring_blocks;
-            const bool smag = c.diffusion == SW_DIFF_SMAGORINSKY;
-            const int rc = launch(ctx, 1, [&] {
-                if (g.ep) tail16_opts<true>(t, o, c.bottom_drag, smag, nb, ctx->stream, ctx->tail_ty);
-                else tail16_opts<false>(t, o, c.bottom_drag, smag, nb, ctx->stream, ctx->tail_ty);
-            });
-            if (rc) return rc;
+            if (e != cudaSuccess) return fail(ctx, SW_ERR_CUDA, std::string("step kernel: ") + cudaGetErrorString(e));
         } else {
-            const int rc = launch(ctx, 5, [&] {
-                s16_pack_uv_kernel<S16><<<4 * ctx->nsm, 256, 0, ctx->stream>>>(
-                    (const float*)ctx->Acc.u, (const float*)ctx->Acc.v, hi[q].u, lo[q].u, hi[q].v, lo[q].v,
-                    (long long)ctx->nelem, s, ctx->dst);
-            });
-            if (rc) return rc;
+            for (int k = 1; k <= c.RKo; k++) {
+                const S16StageArgs<S16> a = stage16_args(ctx, k, p, Fxt, Fyt);
+                const int nblk = (a.nsx * a.nsy + 3) / 4 + a.nring_blocks;
+                const bool first = k == 1, last = k == c.RKo;
+                const int rc = launch(ctx, 0, [&] {
+                    if (g.ep) {
+                        if (first) stage16_ty<true, true, false>(a, nblk, ctx->stream, ctx->stage_ty);
+                        else if (last) stage16_ty<true, false, true>(a, nblk, ctx->stream, ctx->stage_ty);
+                        else stage16_ty<true, false, false>(a, nblk, ctx->stream, ctx->stage_ty);
+                    } else {
+                        if (first) stage16_ty<false, true, false>(a, nblk, ctx->stream, ctx->stage_ty);
+                        else if (last) stage16_ty<false, false, true>(a, nblk, ctx->stream, ctx->stage_ty);
+                        else stage16_ty<false, false, false>(a, nblk, ctx->stream, ctx->stage_ty);
+                    }
+                });
+                if (rc) return rc;
+            }
+
+            if (tail_now) {
+                const TailArgs<float, float> t = tail16_args(ctx, p);
+                const TailStorePair<S16> o = tail16_out(p);
+                const int nb = (t.nsx * t.nsy + 3) / 4 + t.nring_blocks;
+                const bool smag = c.diffusion == SW_DIFF_SMAGORINSKY;
+                const int rc = launch(ctx, 1, [&] {
+                    if (g.ep) tail16_opts<true>(t, o, c.bottom_drag, smag, nb, ctx->stream, ctx->tail_ty);
+                    else tail16_opts<false>(t, o, c.bottom_drag, smag, nb, ctx->stream, ctx->tail_ty);
+                });
+                if (rc) return rc;
+            } else {
+                const int rc = launch(ctx, 5, [&] {
+                    s16_pack_uv_kernel<S16><<<4 * ctx->nsm, 256, 0, ctx->stream>>>(
+                        (const float*)ctx->Acc.u, (const float*)ctx->Acc.v, hi[q].u, lo[q].u, hi[q].v, lo[q].v,
+                        (long long)ctx->nelem, s, ctx->dst);
+                });
+                if (rc) return rc;
+            }
         }
         ctx->t += c.dtint;
 

@@ -18,6 +18,10 @@ StepPlan step_plan(const Geom& g, int nsm, bool hvar, bool ssp);
 template <class T, bool SSP>
 cudaError_t step_launch(const StepPlan& plan, StepArgs<T> a, bool hvar, bool sad, cudaStream_t stream);
 
+// One step of the 16-bit storage form (Float32 arithmetic, RK, Arakawa-Hsu).
+template <class E>
+cudaError_t step16_launch(const StepPlan& plan, StepArgs<float> a, const Step16<E>& io, bool hvar, cudaStream_t stream);
+
 // A launch over the tiles of up to STEP_BATCH members of an ensemble (Float32,
 // RK, Arakawa-Hsu): members' arguments with their tiles (ntx, nty), their
 // numbers of steps and the global step to run.

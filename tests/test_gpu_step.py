@@ -7,6 +7,7 @@
   launches per stage (themselves pinned to the oracle), at sizes the oracle
   would be slow at.
 * The input of the last right-hand side, which the kernel does not keep.
+* The 16-bit storage form in every tile shape against its launches per stage.
 * A run in blocks of steps against the same run step by step.
 """
 import numpy as np
@@ -80,6 +81,26 @@ def test_tile_heights_against_the_launches_per_stage(shape, rows, monkeypatch):
             assert_bitwise(x, y, f"{name} {kw}")
         for x, y, name in zip(rhs_got, rhs, NAMES):
             assert_bitwise(x, y, f"right-hand side's {name} {kw}")
+
+
+@pytest.mark.parametrize("shape", ["0", "1", "2", "3", "4"])
+@pytest.mark.parametrize("storage", ["bf16", "f16"])
+def test_16bit_storage_against_the_launches_per_stage(storage, shape, monkeypatch):
+    """The stored halves and the tracer; α = 0.5 keeps the launches per stage
+    (its ghost increments are rounded on their own)."""
+    options = [kw for kw in OPTIONS if kw.get("T") is None] + [dict(bc="nonperiodic", α=0.0), dict(nstep_diff=2)]
+    for kw in options:
+        for nx, ratio in ((61, 3), (125, 2), (211, 2)):
+            S, Prog = setup(dict(kw, nx=nx, L_ratio=ratio))
+            got = []
+            for step in ("-1", shape):
+                monkeypatch.setenv("SWB200_STEP", step)
+                with Model(S, storage=storage, storage_scale_uv=8.0) as m:
+                    m.set_state(Prog)
+                    assert m.run(3).code == 0
+                    got.append(m.get_state())
+            for x, y, name in zip(*got, NAMES):
+                assert_bitwise(x, y, f"{name} {kw}")
 
 
 @pytest.mark.parametrize("kw", [dict(nx=100), dict(nx=64, Uadv=0.25), dict(nx=64, time_scheme="SSPRK3"),
