@@ -103,15 +103,16 @@ def test_16bit_storage_against_the_launches_per_stage(storage, shape, monkeypatc
                 assert_bitwise(x, y, f"{name} {kw}")
 
 
+@pytest.mark.parametrize("n", [150, 60])   # 16-step blocks, then 4; single steps, then 16, 8 and 4
 @pytest.mark.parametrize("kw", [dict(nx=100), dict(nx=64, Uadv=0.25), dict(nx=64, time_scheme="SSPRK3"),
                                 dict(nx=64, bc="nonperiodic", T=np.float64), dict(nx=600, L_ratio=3)])
-def test_blocks_of_steps_equal_single_steps(kw, monkeypatch):
-    """150 steps in one call (blocks, single steps between the NaN checks)
+def test_blocks_of_steps_equal_single_steps(kw, n, monkeypatch):
+    """n steps in one call (blocks, single steps between the NaN checks)
     against the same steps one call each and without graphs."""
     S, Prog = setup(dict(kw, output_dt=0.5))
-    whole = run(S, Prog, 150)
+    whole = run(S, Prog, n)
     monkeypatch.setenv("SWB200_GRAPHS", "0")
-    single = run(S, Prog, 150)
+    single = run(S, Prog, n)
     for a, b in zip(whole, single):
         for x, y, name in zip(a, b, NAMES):
             assert_bitwise(x, y, name)
