@@ -42,8 +42,11 @@ L2_FLUSH = 256 << 20
 STAGE_BYTES_PER_CELL = (44 + 68 + 68 + 44) / 4
 STEP_BYTES_PER_CELL = 264
 # algorithmic bytes per cell of a whole-step launch (stages and tail in one
-# kernel): reads u, v, eta, H, Fx, writes u, v, eta
+# kernel): reads u, v, eta, H, Fx, writes u, v, eta; in the 16-bit storage form
+# the same as pairs of 16-bit values.  The tracer reads u, v, sst and writes
+# sst: 16 B, or 8 B in 16-bit storage
 WHOLE_STEP_BYTES_PER_CELL = 32
+TRACER_BYTES_PER_CELL, TRACER_BYTES_PER_CELL_16 = 16, 8
 # the 16-bit storage form (scaled 16-bit state pairs, stage increments and
 # accumulated increments; FP32 X0 after the last stage): stage 1 reads the
 # state's pair and writes the stage increment and D (32 B with H, Fx), stages
@@ -450,7 +453,13 @@ def main():
     stage_bytes = STAGE_BYTES_PER_CELL if storage == "native" else STAGE_BYTES_PER_CELL_16
     if main["whole"]:
         stage_bytes = WHOLE_STEP_BYTES_PER_CELL
-    step_bytes = STEP_BYTES_PER_CELL if storage == "native" else STEP_BYTES_PER_CELL_16
+
+    def bytes_of_step(stg, whole):
+        if whole:
+            return WHOLE_STEP_BYTES_PER_CELL + (TRACER_BYTES_PER_CELL if stg == "native" else TRACER_BYTES_PER_CELL_16)
+        return STEP_BYTES_PER_CELL if stg == "native" else STEP_BYTES_PER_CELL_16
+
+    step_bytes = bytes_of_step(storage, main["whole"])
     achieved = stage_bytes * cells / (main["stage_ms"] / 1e3) / 1e9
     peak, peak_kind = peaks()
     # the other forms of the metric on the same workload: the FMA build, and
@@ -465,7 +474,7 @@ def main():
             r = time_form(stg, bld)
             others[name] = {"value": r["value"], "ratio_to_value": r["value"] / value,
                             "ms_per_step": 1e3 * r["t_dev"] / args.steps,
-                            "bytes_per_cell_step": STEP_BYTES_PER_CELL if stg == "native" else STEP_BYTES_PER_CELL_16,
+                            "bytes_per_cell_step": bytes_of_step(stg, r["whole"]),
                             "kernels_us": {k: round(v["avg_us"], 2) for k, v in r["kernels"].items()}}
 
     # e2e: drop-in call with pinned host buffers (create, upload, run, download)

@@ -202,7 +202,9 @@ int sw_get_state(sw_ctx* ctx, void* u, void* v, void* eta, void* sst);
  * the current state before any step.  The reference's output writes q and the
  * relative vorticity from its work arrays (src/output.jl:105-115), which hold
  * the values of that evaluation (src/PV_advection.jl:2-18, src/rhs.jl:89-128);
- * they follow from this state, H and f_q.  Native storage only. */
+ * they follow from this state, H and f_q.  Where a step is one launch that
+ * input is formed again from the step's start when this call asks for it.
+ * Native storage only. */
 int sw_get_rhs_input(sw_ctx* ctx, void* u, void* v, void* eta);
 /* FP64 reductions over the current state. */
 int sw_diagnostics(sw_ctx* ctx, sw_diag* out);
@@ -266,7 +268,8 @@ int sw_batch_run(sw_batch* b, int64_t nsteps, sw_status* statuses);
 int sw_batch_get_state(sw_batch* b, int32_t member, void* u, void* v, void* eta, void* sst);
 int64_t sw_batch_launches(const sw_batch* b);
 /* Rows per warp strip of the batched stage and tail kernels: 4, 8, 16 or 32,
- * or 0 before the first run that could choose.  sw_batch_run chooses it on
+ * or 0 before the first run that could choose; 32 where every member's stages
+ * and tail run as one launch, which has no strips.  sw_batch_run chooses it on
  * its first call of more than 44 global steps: each candidate advances 2
  * untimed steps, then 3 interleaved rounds time 3 steps of each (real steps
  * of the run: every candidate computes identical values) and the best round
