@@ -35,11 +35,11 @@
 // 23.8 -> 22.4.  The stop flag is read beside the state.
 //
 // Measured (B200, us per step with the tracer beside it; the four stage
-// launches and the tail before): 64x32 24.5 -> 10.7, 256x128 26.3 -> 11.8,
-// 512x256 49.9 -> 21.5, 1000x500 over a ridge 89 -> 38.5, 2048x1024 181 -> 125,
-// 512x256 Float64 60 -> 25.6, SSPRK3 500x250 42.4 -> 27.5.  The 103 x 47 tile
-// of 63 rows takes 65 thousand clocks: load 6, A 4 x 4.2, B 4 x 7.5, T1 5, T2
-// 7.5, the rest start and end.  A third of the issue slots are used (sixteen
+// launches and the tail before): 64x32 22.6 -> 10.0, 256x128 25.6 -> 10.8,
+// 512x256 48.7 -> 19.6, 1000x500 over a ridge 88 -> 37.8, 2048x1024 181 -> 123,
+// 512x256 Float64 60 -> 23.1, SSPRK3 500x250 41.8 -> 26.0.  The 103 x 47 tile
+// of 63 rows takes 65 thousand clocks: load 6, A 4 x 4.2, B 4 x 7.5, T1 and
+// T2 11, the rest start and end.  A third of the issue slots are used (sixteen
 // warps of 128 registers); a warp waits most for the fixed latency of its
 // packed adds, then for barriers, loads and the shared memory about equally.
 // 20, 24 and 32 warps with fewer registers, passes A, T1 and T2 unrolled by 4
@@ -180,6 +180,21 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, const IO& io, ty
     const int EHv = zy1 - zy;                             // rows of this tile
     const P half = A.half, q4 = A.q4, nz = A.nz;
     const bool lowwall = zy == -2, highwall = zy1 == M + 2;
+
+    // This warp's rows of [from, to) in the passes that keep nothing in registers from one to the next: an equal share,
+    // as the rows shrink from stage to stage and a tile's outputs are half to three quarters of its rows (512x256 21.5
+    // -> 19.6 us a step, 2048x1024 125 -> 122.7, SSPRK3 200x100 Float64 26.7 -> 19.8).  With one row per thread its own,
+    // which is known not to loop (64x32 10.1 against 11.3).
+    auto share = [&](int from, int to, int& r0, int& r1) {
+        if constexpr (R == 1) {
+            r0 = max(ly0, from);
+            r1 = min(ly0 + 1, to);
+        } else {
+            const int n = (to - from + SH::NG - 1) / SH::NG;
+            r0 = from + warp / SH::EWW * n;
+            r1 = min(r0 + n, to);
+        }
+    };
 
     // this thread's columns
     int X[V];
@@ -409,7 +424,8 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, const IO& io, ty
         // ---- pass A: q, U, V, p
         {
             const P gg = A.g_;
-            const int r0 = max(ly0, a0), r1 = min(ly0 + R, a1);
+            int r0, r1;
+            share(a0, a1, r0, r1);
             if (r0 < r1) {
                 int s = r0 * EW + lx;
                 P u_m = su[s - EW], v_c = sv[s], h_m, hs_m;
@@ -599,7 +615,8 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, const IO& io, ty
             const int sub = A.sub[k];
             const bool mix = k == A.combo, needX = mix || sub == STEP_KN;
             const int dX = EDGE ? X[V - 1] - X[0] : (V - 1) * SHIFT;
-            const int r0 = max(ly0, lowwall ? -zy : ay + 1), r1 = min(ly0 + R, highwall ? M - zy : by - 1);
+            int r0, r1;
+            share(lowwall ? -zy : ay + 1, highwall ? M - zy : by - 1, r0, r1);
             // e at EW-2 and EW-1 of the lower half come from the upper half's lanes 2, 3
             const bool prod_e = V == 1 || (lx >= 2 && lx <= EW - 3), xch_e = V == 2 && (xch || lx == 2);
             const int xofs_e = lx <= 3 ? 2 * SHIFT : -2 * SHIFT + 1;
@@ -653,7 +670,8 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, const IO& io, ty
     // ---- tail.  T1: ν (sq), Lu (sU), Lv (sV), sqrt(KE) (sp) on the tile and one point around it
     const bool quad = A.drag == SW_DRAG_QUADRATIC, smag = A.smag != 0;
     if (A.tail) {
-        const int r0 = max(ly0, max(ys - 1 - zy, lowwall ? 1 : 0)), r1 = min(ly0 + R, ye + 1 - zy);
+        int r0, r1;
+        share(max(ys - 1 - zy, lowwall ? 1 : 0), ye + 1 - zy, r0, r1);
         if (r0 < r1) {
             const P cS = A.cSmag;
             int s = r0 * EW + lx;
@@ -695,7 +713,8 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, const IO& io, ty
     // ---- T2: the new u, v, eta of the tile (and its untouched halo cells)
     {
         const int t0 = ys == 0 ? -2 : ys, t1 = ye == M ? M + 2 : ye;
-        const int r0 = max(ly0, t0 - zy), r1 = min(ly0 + R, t1 - zy);
+        int r0, r1;
+        share(t0 - zy, t1 - zy, r0, r1);
         if (r0 < r1) {
             const P cD = A.cD, rD = A.rD, Dt = A.Dt_diff, nuB = A.nuB;
             int s = r0 * EW + lx;
@@ -739,10 +758,12 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, const IO& io, ty
                         const P Hc = HVAR ? sH[s] : tH[ly];
                         const P h = K::add(se[s], Hc), hl = K::add(se[s - 1], HVAR ? sH[s - 1] : Hc);
                         const P sK = sp[s];
-                        Bu = K::div(K::mulx(K::mulx(cD, K::mulx(half, K::add(sK, sp[s - 1]))), u_c),
-                                    K::mulx(half, K::add(h, hl)));
-                        Bv = K::div(K::mulx(K::mulx(cD, K::mulx(half, K::add(sK, sK_m))), v_c),
-                                    K::mulx(half, K::add(h, h_m)));
+                        if (!EDGE || R == 1 || (y >= 0 && y < M)) {   // elsewhere u and v keep theirs, and h may be zero
+                            Bu = K::div(K::mulx(K::mulx(cD, K::mulx(half, K::add(sK, sp[s - 1]))), u_c),
+                                        K::mulx(half, K::add(h, hl)));
+                            Bv = K::div(K::mulx(K::mulx(cD, K::mulx(half, K::add(sK, sK_m))), v_c),
+                                        K::mulx(half, K::add(h, h_m)));
+                        }
                         h_m = h; sK_m = sK;
                     } else if (A.drag == SW_DRAG_LINEAR) {
                         Bu = K::mul(rD, u_c, nz);

@@ -13,12 +13,12 @@ namespace {
 
 // Tile shapes (StepShape: warps side by side, warps, rows per thread).  Low
 // tiles for grids that leave SMs idle: a pass is then one row's latency, and
-// more rows per block cost more clocks than their halos (64x32: 20 rows 10.7 us
-// a step, 24 11.2, 32 12.3; 256x128 needs 24 rows to run in one wave, 11.8
-// against 19.8).  32 rows fill the gap up to 512x256 (400x200: 14.7, else
-// 19.0), 2 warps side by side the ones above (512x256: 21.5 against 23.4).
+// more rows per block cost more clocks than their halos (64x32: 20 rows 10.0 us
+// a step, 24 10.5, 32 11.6; 256x128 needs 24 rows to run in one wave, 10.8
+// against 18.6).  32 rows fill the gap up to 512x256 (400x200: 13.5, else
+// 15.7), 2 warps side by side the ones above (512x256: 19.6 against 22.2).
 // The last shape fills the shared memory of an SM, for several waves
-// (2048x1024: 125 against 171); with a depth that varies along x the eighth
+// (2048x1024: 123 against 164); with a depth that varies along x the eighth
 // array costs it rows.
 template <class T, bool HVAR>
 struct Shapes;
