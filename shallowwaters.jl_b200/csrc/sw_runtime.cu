@@ -235,6 +235,9 @@ struct sw_ctx {
     int stage_blocks_cap = 0;     // > 0: at most this many persistent blocks in rk_stage_tma
     uint32_t spin_limit = MBAR_SPIN_LIMIT;   // polls per bounded wait of rk_stage_tma
     int test_skip_chunk = -1;     // test only: a chunk rk_stage_tma's producer leaves out
+    // test only: n > 0: the n-th kernel launch from here on reports an error and is not issued
+    int test_fail_launch = 0;
+    bool refused() { return test_fail_launch > 0 && --test_fail_launch == 0; }
     // CUDA graphs of one time step, keyed by the buffer parities and the
     // sub-steps that are due (see step_key); off with SWB200_GRAPHS=0
     bool use_graphs = true;
@@ -386,6 +389,7 @@ int launch(sw_ctx* ctx, int kind, F&& f) {
         b = ctx->evget();
         cudaEventRecord(a, ctx->stream);
     }
+    if (ctx->refused()) return fail(ctx, SW_ERR_CUDA, "kernel launch: refused for a test");
     f();
     ctx->launches++;
     cudaError_t e = cudaGetLastError();
@@ -1777,7 +1781,7 @@ std::string env_settings() {
     std::string s;
     for (const char* k : {"SWB200_TMA", "SWB200_GRAPHS", "SWB200_STAGE_BLOCKS", "SWB200_TAIL_TY", "SWB200_STAGE_TY",
                           "SWB200_STEP", "SWB200_STEP_ROWS",
-                          "SWB200_TEST_WAIT_LIMIT", "SWB200_TEST_SKIP_CHUNK"}) {
+                          "SWB200_TEST_WAIT_LIMIT", "SWB200_TEST_SKIP_CHUNK", "SWB200_TEST_FAIL_LAUNCH"}) {
         const char* v = getenv(k);
         s += k;
         s += '=';
@@ -2199,9 +2203,11 @@ int batch_build(sw_batch* b) {
 }
 
 // the launches of group gr for a global step of parity p (the step read from
-// b->d_step), on stream s; returns how many
+// b->d_step), on stream s; returns how many.  e: the error of a whole-step
+// launch that was refused (a capture does not show it: the graph would hold
+// a step without its stages)
 template <bool PER, int TY>
-int batch_group_step(sw_batch* b, const BatchGroup& gr, int p, cudaStream_t s, int ti) {
+int batch_group_step(sw_batch* b, const BatchGroup& gr, int p, cudaStream_t s, int ti, cudaError_t& e) {
     const int n = (int)gr.idx.size();
     const long long* i = b->d_step;
     int launches = 0;
@@ -2220,7 +2226,8 @@ int batch_group_step(sw_batch* b, const BatchGroup& gr, int p, cudaStream_t s, i
                 sb->m[q].nty = gr.plans[m0 + q].nty;
                 sb->nt[q] = ctx->cfg.nt;
             }
-            (void)step_batch_launch(gr.step_shape, *sb, s);    // a failure shows at the capture's end
+            e = b->mem[gr.idx[m0]]->refused() ? cudaErrorLaunchOutOfResources : step_batch_launch(gr.step_shape, *sb, s);
+            if (e != cudaSuccess) return launches;
             launches++;
         }
     } else {
@@ -2302,19 +2309,19 @@ int batch16_group_step(sw_batch* b, const BatchGroup& gr, int p, cudaStream_t s,
 }
 
 template <bool PER, int TY>
-int batch_group_step_storage(sw_batch* b, const BatchGroup& gr, int p, cudaStream_t s, int ti) {
+int batch_group_step_storage(sw_batch* b, const BatchGroup& gr, int p, cudaStream_t s, int ti, cudaError_t& e) {
     if (gr.storage == SW_STORE_BF16) return batch16_group_step<__nv_bfloat16, PER, TY>(b, gr, p, s, ti);
     if (gr.storage == SW_STORE_F16) return batch16_group_step<__half, PER, TY>(b, gr, p, s, ti);
-    return batch_group_step<PER, TY>(b, gr, p, s, ti);
+    return batch_group_step<PER, TY>(b, gr, p, s, ti, e);
 }
 
 template <bool PER>
-int batch_group_step_ty(sw_batch* b, const BatchGroup& gr, int p, cudaStream_t s, int ti) {
+int batch_group_step_ty(sw_batch* b, const BatchGroup& gr, int p, cudaStream_t s, int ti, cudaError_t& e) {
     switch (BATCH_TYS[ti]) {
-        case 4: return batch_group_step_storage<PER, 4>(b, gr, p, s, ti);
-        case 8: return batch_group_step_storage<PER, 8>(b, gr, p, s, ti);
-        case 16: return batch_group_step_storage<PER, 16>(b, gr, p, s, ti);
-        default: return batch_group_step_storage<PER, 32>(b, gr, p, s, ti);
+        case 4: return batch_group_step_storage<PER, 4>(b, gr, p, s, ti, e);
+        case 8: return batch_group_step_storage<PER, 8>(b, gr, p, s, ti, e);
+        case 16: return batch_group_step_storage<PER, 16>(b, gr, p, s, ti, e);
+        default: return batch_group_step_storage<PER, 32>(b, gr, p, s, ti, e);
     }
 }
 
@@ -2329,7 +2336,8 @@ int batch_graph(sw_batch* b, int p, int ti) {
         const BatchGroup& gr = b->groups[g];
         cudaStream_t gs = b->gstreams[g];
         if ((e = cudaStreamWaitEvent(gs, b->events[0], 0)) != cudaSuccess) break;
-        launches += gr.per ? batch_group_step_ty<true>(b, gr, p, gs, ti) : batch_group_step_ty<false>(b, gr, p, gs, ti);
+        launches += gr.per ? batch_group_step_ty<true>(b, gr, p, gs, ti, e) : batch_group_step_ty<false>(b, gr, p, gs, ti, e);
+        if (e != cudaSuccess) break;
         if ((e = cudaEventRecord(b->events[g + 1], gs)) != cudaSuccess) break;
         e = cudaStreamWaitEvent(s, b->events[g + 1], 0);
     }
@@ -2344,6 +2352,7 @@ int batch_graph(sw_batch* b, int p, int ti) {
     if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph[ti][p], graph, 0);
     if (graph) cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
+        (void)cudaGetLastError();
         b->err = std::string("batch graph: ") + cudaGetErrorString(e);
         return SW_ERR_CUDA;
     }
@@ -2676,6 +2685,9 @@ int sw_create(const sw_config* cfg, const sw_static* st, sw_ctx** out) {
         if (envw && atoi(envw) > 0) ctx->spin_limit = (uint32_t)atoi(envw);
         const char* envk = getenv("SWB200_TEST_SKIP_CHUNK");
         ctx->test_skip_chunk = envk ? atoi(envk) : -1;
+        // test only: a launch that fails on the host
+        const char* envl = getenv("SWB200_TEST_FAIL_LAUNCH");
+        ctx->test_fail_launch = envl ? atoi(envl) : 0;
         for (Fields3* f : {&ctx->S[0], &ctx->S[1], &ctx->A, &ctx->B, &ctx->Acc})
             for (void* p : {f->u, f->v, f->e}) {
                 if (!ok) break;
