@@ -232,6 +232,7 @@ struct sw_ctx {
     TileSched* sched = nullptr;   // device tile counter of the TMA stage kernel
     std::map<const void*, Maps> tmaps;
     bool use_tma = false;
+    std::map<const void*, int> tma_blocks;   // per TMA stage kernel prepared for this context: its blocks per SM
     int stage_blocks_cap = 0;     // > 0: at most this many persistent blocks in rk_stage_tma
     uint32_t spin_limit = MBAR_SPIN_LIMIT;   // polls per bounded wait of rk_stage_tma
     int test_skip_chunk = -1;     // test only: a chunk rk_stage_tma's producer leaves out
@@ -509,7 +510,13 @@ struct Engine : EngineBase {
         const sw_config& c = ctx->cfg;
         if (!step_launches(ctx)) return SW_OK;
         if constexpr (STEP_TYPES)
-            if (step_fits(ctx)) ctx->step_plan = step_plan<T>(ctx->g, ctx->nsm, ctx->H.sx != 0, c.time_scheme != SW_RK);
+            if (step_fits(ctx)) {
+                const bool hvar = ctx->H.sx != 0, sad = c.adv_scheme == SW_SADOURNY;
+                ctx->step_plan = step_plan<T>(ctx->g, ctx->nsm, hvar, c.time_scheme != SW_RK);
+                if (ctx->step_plan.shape >= 0)
+                    CK((c.time_scheme == SW_RK ? step_prepare<T, false>(ctx->step_plan, hvar, sad)
+                                               : step_prepare<T, true>(ctx->step_plan, hvar, sad)));
+            }
         return SW_OK;
     }
 
@@ -573,14 +580,11 @@ struct Engine : EngineBase {
         constexpr int TY = STAGE_TMA_TY, K = STAGE_TMA_K, S = STAGE_TMA_S;
         auto kern = rk_stage_tma<T, Tp, PER, FIRST, LAST, TY, K, S, ROWF>;
         constexpr int smem = stage_tma_smem<T, Tp, FIRST, LAST, K, S>();
-        // per instantiation, set up once and thread-safely
-        static const int occ = [&] {
-            int o = -1;
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, 160, smem) != cudaSuccess)
-                o = -1;
-            return o;
-        }();
+        // set up once per context: the shared-memory limit belongs to the device and the CUDA context
+        int& occ = ctx->tma_blocks[(const void*)kern];
+        if (occ < 1 && (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+                        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 160, smem) != cudaSuccess))
+            occ = 0;
         if (occ < 1) return -1;
         const Geom& g = a.g;
         const int ntiles = ((g.N + BAND - 1) / BAND) * ((g.M + TY - 1) / TY);
@@ -1174,8 +1178,10 @@ struct Engine16 : Engine<float, float> {
         // The whole-step kernel, where a ghost point's rounded increment is its source's (copies
         // and (1-α) = ±1: a rounded multiple is not the multiple of the rounded otherwise).
         if (this->step_launches(ctx) && this->step_fits(ctx) &&
-            (c.periodic || c.one_minus_alpha == 1.0 || c.one_minus_alpha == -1.0))
+            (c.periodic || c.one_minus_alpha == 1.0 || c.one_minus_alpha == -1.0)) {
             ctx->step_plan = step_plan<float>(ctx->g, ctx->nsm, ctx->H.sx != 0, false);
+            if (ctx->step_plan.shape >= 0) CK(step16_prepare<S16>(ctx->step_plan, ctx->H.sx != 0));
+        }
         return SW_OK;
     }
 
@@ -2140,6 +2146,7 @@ int batch_build(sw_batch* b) {
             }
             gr.plans.resize(n);
             if (fits) gr.step_shape = step_batch_plan(gs.data(), n, b->mem[gr.idx[0]]->nsm, gr.plans.data());
+            if (gr.step_shape >= 0 && step_batch_prepare(gr.step_shape) != cudaSuccess) return SW_ERR_CUDA;
         }
         std::vector<int> cs[BATCH_NTY], ct[BATCH_NTY], ctr, nbx, cc, cn;
         std::vector<BatchMember> mems;

@@ -27,12 +27,20 @@ __global__ void __launch_bounds__(SH::NW * 32, 1) rk_step_batch(const __grid_con
 }
 
 template <class SH>
-cudaError_t go_batch(const StepBatch& b, int nblocks, cudaStream_t stream) {
+cudaError_t go_batch(const StepBatch* b, int nblocks, cudaStream_t stream) {
     constexpr int smem = SH::smem(true);
-    static const cudaError_t e = cudaFuncSetAttribute(rk_step_batch<SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    rk_step_batch<SH><<<nblocks, SH::NW * 32, smem, stream>>>(b);
+    if (!b) return cudaFuncSetAttribute(rk_step_batch<SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    rk_step_batch<SH><<<nblocks, SH::NW * 32, smem, stream>>>(*b);
     return cudaGetLastError();
+}
+
+cudaError_t go_batch_shape(int shape, const StepBatch* b, int nblocks, cudaStream_t stream) {
+    using SS = Shapes<float, true>;
+    if (shape == 0) return go_batch<SS::S0>(b, nblocks, stream);
+    if (shape == 1) return go_batch<SS::S1>(b, nblocks, stream);
+    if (shape == 2) return go_batch<SS::S2>(b, nblocks, stream);
+    if (shape == 3) return go_batch<SS::S3>(b, nblocks, stream);
+    return go_batch<SS::S4>(b, nblocks, stream);
 }
 
 // a member's tiles in shape s with at most h rows each; false if it has none
@@ -77,19 +85,15 @@ int step_batch_plan(const Geom* gs, int n, int nsm, StepPlan* plans) {
     return best;
 }
 
+cudaError_t step_batch_prepare(int shape) { return go_batch_shape(shape, nullptr, 0, nullptr); }
+
 cudaError_t step_batch_launch(int shape, StepBatch& b, cudaStream_t stream) {
-    using SS = Shapes<float, true>;
     b.block0[0] = 0;
     for (int m = 0; m < b.n; m++) {
         set_constants<float, false>(b.m[m]);
         b.block0[m + 1] = b.block0[m] + b.m[m].ntx * b.m[m].nty;
     }
-    const int nb = b.block0[b.n];
-    if (shape == 0) return go_batch<SS::S0>(b, nb, stream);
-    if (shape == 1) return go_batch<SS::S1>(b, nb, stream);
-    if (shape == 2) return go_batch<SS::S2>(b, nb, stream);
-    if (shape == 3) return go_batch<SS::S3>(b, nb, stream);
-    return go_batch<SS::S4>(b, nb, stream);
+    return go_batch_shape(shape, &b, b.block0[b.n], stream);
 }
 
 }  // namespace swb

@@ -107,17 +107,18 @@ cudaError_t go_prepared(Kernel kern, int smem, int nblocks, cudaStream_t stream,
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// without arguments: allows the kernel its shared memory in the current CUDA context
 template <class T, class S, bool HVAR, bool SSP, bool SAD>
-cudaError_t go(const StepArgs<T>& a, cudaStream_t stream) {
+cudaError_t go(const StepArgs<T>* a, cudaStream_t stream) {
     auto kern = rk_step_kernel<T, S, HVAR, SSP, SAD>;
     constexpr int smem = S::smem(HVAR);
     static_assert(smem <= 227 * 1024, "tile beyond the shared memory of an SM");
-    static const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return e != cudaSuccess ? e : go_prepared<S>(kern, smem, a.ntx * a.nty, stream, a);
+    if (!a) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return go_prepared<S>(kern, smem, a->ntx * a->nty, stream, *a);
 }
 
 template <class T, bool HVAR, bool SSP, bool SAD>
-cudaError_t go_shape(int shape, const StepArgs<T>& a, cudaStream_t stream) {
+cudaError_t go_shape(int shape, const StepArgs<T>* a, cudaStream_t stream) {
     using SS = Shapes<T, HVAR>;
     if (shape == 0) return go<T, typename SS::S0, HVAR, SSP, SAD>(a, stream);
     if (shape == 1) return go<T, typename SS::S1, HVAR, SSP, SAD>(a, stream);
@@ -146,12 +147,22 @@ void set_constants(StepArgs<T>& a) {
 }
 
 template <class T, bool SSP>
+cudaError_t go_variant(int shape, const StepArgs<T>* a, bool hvar, bool sad, cudaStream_t stream) {
+    if (hvar) return sad ? go_shape<T, true, SSP, true>(shape, a, stream) : go_shape<T, true, SSP, false>(shape, a, stream);
+    return sad ? go_shape<T, false, SSP, true>(shape, a, stream) : go_shape<T, false, SSP, false>(shape, a, stream);
+}
+
+template <class T, bool SSP>
+cudaError_t step_prepare(const StepPlan& p, bool hvar, bool sad) {
+    return go_variant<T, SSP>(p.shape, nullptr, hvar, sad, nullptr);
+}
+
+template <class T, bool SSP>
 cudaError_t step_launch(const StepPlan& p, StepArgs<T> a, bool hvar, bool sad, cudaStream_t stream) {
     a.ntx = p.ntx;
     a.nty = p.nty;
     set_constants<T, SSP>(a);
-    if (hvar) return sad ? go_shape<T, true, SSP, true>(p.shape, a, stream) : go_shape<T, true, SSP, false>(p.shape, a, stream);
-    return sad ? go_shape<T, false, SSP, true>(p.shape, a, stream) : go_shape<T, false, SSP, false>(p.shape, a, stream);
+    return go_variant<T, SSP>(p.shape, &a, hvar, sad, stream);
 }
 
 }  // namespace swb

@@ -18,15 +18,15 @@ s16_step_kernel(const __grid_constant__ StepArgs<float> A, const __grid_constant
 }
 
 template <class SH, bool HVAR, class E>
-cudaError_t go16(const StepArgs<float>& a, const Step16<E>& io, cudaStream_t stream) {
+cudaError_t go16(const StepArgs<float>* a, const Step16<E>& io, cudaStream_t stream) {
     auto kern = s16_step_kernel<SH, HVAR, E>;
     constexpr int smem = SH::smem(HVAR);
-    static const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return e != cudaSuccess ? e : go_prepared<SH>(kern, smem, a.ntx * a.nty, stream, a, io);
+    if (!a) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return go_prepared<SH>(kern, smem, a->ntx * a->nty, stream, *a, io);
 }
 
 template <bool HVAR, class E>
-cudaError_t go16_shape(int shape, const StepArgs<float>& a, const Step16<E>& io, cudaStream_t stream) {
+cudaError_t go16_shape(int shape, const StepArgs<float>* a, const Step16<E>& io, cudaStream_t stream) {
     using SS = Shapes<float, HVAR>;
     if (shape == 0) return go16<typename SS::S0, HVAR>(a, io, stream);
     if (shape == 1) return go16<typename SS::S1, HVAR>(a, io, stream);
@@ -42,8 +42,17 @@ cudaError_t step16_launch(const StepPlan& p, StepArgs<float> a, const Step16<E>&
     a.ntx = p.ntx;
     a.nty = p.nty;
     set_constants<float, false>(a);
-    return hvar ? go16_shape<true>(p.shape, a, io, stream) : go16_shape<false>(p.shape, a, io, stream);
+    return hvar ? go16_shape<true>(p.shape, &a, io, stream) : go16_shape<false>(p.shape, &a, io, stream);
 }
+
+template <class E>
+cudaError_t step16_prepare(const StepPlan& p, bool hvar) {
+    const Step16<E> io{};
+    return hvar ? go16_shape<true>(p.shape, nullptr, io, nullptr) : go16_shape<false>(p.shape, nullptr, io, nullptr);
+}
+
+template cudaError_t step16_prepare<__nv_bfloat16>(const StepPlan&, bool);
+template cudaError_t step16_prepare<__half>(const StepPlan&, bool);
 
 template cudaError_t step16_launch(const StepPlan&, StepArgs<float>, const Step16<__nv_bfloat16>&, bool, cudaStream_t);
 template cudaError_t step16_launch(const StepPlan&, StepArgs<float>, const Step16<__half>&, bool, cudaStream_t);

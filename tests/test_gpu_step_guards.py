@@ -1,7 +1,13 @@
 """What the whole-step kernel's callers promise beside its values
-(tests/test_gpu_step.py): a refused launch is an error."""
+(tests/test_gpu_step.py): a refused launch is an error; any CUDA context of
+the process may use them."""
+import os
+import subprocess
+import sys
+
 import pytest
 
+from conftest import REPO
 from swb200 import abi
 from swb200.ensemble import Member, _batch_create, run_batched
 
@@ -27,3 +33,51 @@ def test_a_refused_batch_launch_fails_the_run(nth, monkeypatch):
     monkeypatch.delenv("SWB200_TEST_FAIL_LAUNCH")
     rows = run_batched(members(2))
     assert all(r[3] == 0 for r in rows.values())
+
+
+SECOND_CONTEXT = """
+import ctypes as C, os, sys
+import numpy as np
+from swb200 import Model, Parameter, initial_conditions, model_setup
+from swb200.ensemble import Member, run_batched
+
+RUNS = [dict(nx=512), dict(nx=200, T=np.float64, topography="seamount"), dict(nx=128, time_scheme="SSPRK3"),
+        dict(nx=64, adv_scheme="Sadourny", topography="flat"), dict(nx=128, storage="bf16"), dict(nx=128, storage="f16"),
+        dict(nx=256, env=dict(SWB200_TMA="1"))]
+
+def everything():
+    out = []
+    for kw in RUNS:
+        kw = dict(kw)
+        storage, env = kw.pop("storage", "native"), kw.pop("env", {})
+        P = Parameter(**{**dict(Ndays=1.0, Uadv=1000, initial_cond="rest"), **kw})
+        S = model_setup(P)
+        eta = np.random.default_rng(1).normal(0, 0.01, (S.grid.ny, S.grid.nx))
+        os.environ.update(env)
+        with Model(S, storage=storage) as m:
+            m.set_state(initial_conditions(P.Tprog, S, η0=eta))
+            assert m.run(3).code == 0
+            out += list(m.get_state())
+        for k in env:
+            del os.environ[k]
+    _, final = run_batched([Member(k, dict(nx=[48, 200][k], Ndays=0.1), seed=k) for k in range(2)], return_states=True)
+    return out + [f for k in sorted(final) for f in final[k]]
+
+first = everything()
+cu = C.CDLL("libcuda.so.1")
+dev, ctx = C.c_int(), C.c_void_p()
+assert cu.cuDeviceGet(C.byref(dev), 0) == 0 and cu.cuCtxCreate_v2(C.byref(ctx), 0, dev) == 0
+second = everything()
+assert len(first) == len(second) > 0
+for k, (a, b) in enumerate(zip(first, second)):
+    assert np.isfinite(a).all() and np.array_equal(a, b), k
+print("equal")
+"""
+
+
+def test_a_second_cuda_context_in_the_process():
+    """The shared memory that the kernels ask for is allowed per device and
+    CUDA context, so a process may use the library in several."""
+    r = subprocess.run([sys.executable, "-c", SECOND_CONTEXT], capture_output=True, text=True, timeout=300,
+                       env={**os.environ, "PYTHONPATH": os.path.join(REPO, "shallowwaters.jl_b200")})
+    assert r.returncode == 0 and "equal" in r.stdout, r.stderr[-2000:]
