@@ -978,23 +978,24 @@ struct Engine : EngineBase {
 
     // The input of the last step's last stage, formed again by the launches of
     // its earlier stages (the same values) from the state the step started
-    // from.  A NaN stop would make them return at once: it is lifted meanwhile.
+    // from.  A NaN stop would make them return at once: it is lifted meanwhile,
+    // and back in place whether they succeed or not.
     int rhs_again(sw_ctx* ctx) override {
         if (ctx->rhs_in.u || ctx->rhs_p < 0) return SW_OK;
         T Fxt, Fyt;
         wind_factors(ctx, ctx->rhs_t, Fxt, Fyt);
         CK(cudaMemcpyAsync(ctx->hst, ctx->dst, sizeof(DevStatus), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaMemsetAsync(ctx->dst, 0, sizeof(DevStatus), ctx->stream));
+        int rc = SW_OK;
         if (ctx->cfg.time_scheme == SW_RK) {
-            for (int k = 1; k < ctx->cfg.RKo; k++)
-                if (int rc = rk_stage(ctx, k, ctx->rhs_p, true, Fxt, Fyt)) return rc;
-            ctx->rhs_in = (ctx->cfg.RKo % 2 == 0) ? ctx->A : ctx->B;
+            for (int k = 1; k < ctx->cfg.RKo && !rc; k++) rc = rk_stage(ctx, k, ctx->rhs_p, true, Fxt, Fyt);
+            if (!rc) ctx->rhs_in = (ctx->cfg.RKo % 2 == 0) ? ctx->A : ctx->B;
         } else {
             // all sub-stages but the last write stage buffers only; ssp_stages records the last one's input
-            if (int rc = ssp_stages(ctx, ctx->S[ctx->rhs_p], ctx->S[1 - ctx->rhs_p], true, Fxt, Fyt, true)) return rc;
+            rc = ssp_stages(ctx, ctx->S[ctx->rhs_p], ctx->S[1 - ctx->rhs_p], true, Fxt, Fyt, true);
         }
         CK(cudaMemcpyAsync(ctx->dst, ctx->hst, sizeof(DevStatus), cudaMemcpyHostToDevice, ctx->stream));
-        return SW_OK;
+        return rc;
     }
 
     int step(sw_ctx* ctx, long long i) override {

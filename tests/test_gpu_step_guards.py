@@ -5,10 +5,11 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 
-from conftest import REPO
-from swb200 import abi
+from conftest import REPO, assert_bitwise, seeded_inputs
+from swb200 import Model, Parameter, abi, initial_conditions, model_setup
 from swb200.ensemble import Member, _batch_create, run_batched
 
 pytestmark = pytest.mark.gpu
@@ -81,3 +82,33 @@ def test_a_second_cuda_context_in_the_process():
     r = subprocess.run([sys.executable, "-c", SECOND_CONTEXT], capture_output=True, text=True, timeout=300,
                        env={**os.environ, "PYTHONPATH": os.path.join(REPO, "shallowwaters.jl_b200")})
     assert r.returncode == 0 and "equal" in r.stdout, r.stderr[-2000:]
+
+
+def stopped(kw, monkeypatch, refuse=0):
+    """A context that a NaN check has stopped, and what it holds; the
+    ``refuse``-th of its launches reports an error."""
+    monkeypatch.setenv("SWB200_GRAPHS", "0")          # every launch is the context's own
+    if refuse:
+        monkeypatch.setenv("SWB200_TEST_FAIL_LAUNCH", str(refuse))
+    S = model_setup(Parameter(**{**dict(nx=100, Ndays=2, Uadv=1000, tracer_advection=False, output_dt=0.5), **kw}))
+    Prog = initial_conditions(S.parameters.Tprog, S, **seeded_inputs(S, 5))
+    Prog.u[5, 7] = np.nan
+    m = Model(S)
+    m.set_state(Prog)
+    assert m.run(S.grid.nt).code == abi.SW_NAN_DETECTED
+    return m
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(time_scheme="SSPRK3")])
+def test_a_failed_right_hand_side_leaves_the_stop_in_place(kw, monkeypatch):
+    """sw_get_rhs_input lifts the NaN stop while it runs the earlier stages
+    again; when one of them fails the context is still a stopped one."""
+    with stopped(kw, monkeypatch) as m:
+        n = m.kernel_launches
+    with stopped(kw, monkeypatch, refuse=n + 1) as m:
+        with pytest.raises(abi.SwError):
+            m.get_rhs_input()
+        before = m.get_state()
+        m.run(2)                                       # returns at once: back at the same parity
+        for x, y, name in zip(m.get_state(), before, ("u", "v", "η", "sst")):
+            assert_bitwise(x, y, name)
