@@ -251,6 +251,7 @@ struct sw_ctx {
     // model time rhs_t (-1: no such step)
     int rhs_p = -1;
     long long rhs_t = 0;
+    bool stopped = false;      // a NaN check has failed since the state was set: launches return at once
     StepPlan step_plan;        // tiles of the whole-step kernel (shape < 0: not used)
     // while a block of steps is captured: the branch its tracers run on and
     // their events (see capture_block); null otherwise
@@ -1736,6 +1737,9 @@ int run_steps(sw_ctx* ctx, long long nsteps, sw_status* status) {
     const sw_config& c = ctx->cfg;
     long long done = 0;
     int code = SW_OK;
+    const Fields3 rhs_in = ctx->rhs_in;
+    const int rhs_p = ctx->rhs_p;
+    const long long rhs_t = ctx->rhs_t;
     while (done < nsteps) {
         long long i = ctx->step + 1, ran = 0;
         int rc = do_block(ctx, i, nsteps - done, &ran);
@@ -1744,6 +1748,11 @@ int run_steps(sw_ctx* ctx, long long nsteps, sw_status* status) {
             ran = 1;
         }
         if (rc) return rc;
+        if (ctx->stopped) {         // no right-hand side was evaluated
+            ctx->rhs_in = rhs_in;
+            ctx->rhs_p = rhs_p;
+            ctx->rhs_t = rhs_t;
+        }
         done += ran;
         i += ran - 1;
         bool check = (i % c.nout) == 0;
@@ -1759,6 +1768,7 @@ int run_steps(sw_ctx* ctx, long long nsteps, sw_status* status) {
             if (ctx->hst->stop) {
                 // state stays S[p] (before this step); the tracer already moved sst
                 ctx->step = i;
+                ctx->stopped = true;
                 code = SW_NAN_DETECTED;
                 break;
             }
@@ -1849,6 +1859,7 @@ int state_copy_in(sw_ctx* ctx, const void* u, const void* v, const void* eta, co
     ctx->p = 0; ctx->sp = 0; ctx->step = 0; ctx->t = 0;
     ctx->rhs_in = Fields3();
     ctx->rhs_p = -1;
+    ctx->stopped = false;
     int rc;
     if ((rc = copy_in(ctx, ctx->S[0].u, u, shape_u(ctx->g)))) return rc;
     if ((rc = copy_in(ctx, ctx->S[0].v, v, shape_v(ctx->g)))) return rc;

@@ -112,3 +112,17 @@ def test_a_failed_right_hand_side_leaves_the_stop_in_place(kw, monkeypatch):
         m.run(2)                                       # returns at once: back at the same parity
         for x, y, name in zip(m.get_state(), before, ("u", "v", "η", "sst")):
             assert_bitwise(x, y, name)
+
+
+@pytest.mark.parametrize("step", ["-1", "0"])
+def test_the_right_hand_side_of_a_stopped_context(step, monkeypatch):
+    """Steps asked of a stopped context evaluate nothing: the input of the
+    last right-hand side stays that of the step the check stopped at."""
+    monkeypatch.setenv("SWB200_STEP", step)
+    with stopped({}, monkeypatch) as m:
+        before = m.get_rhs_input()
+    with stopped({}, monkeypatch) as m:
+        for n in (2, 1, 3):
+            m.run(n)
+            for x, y, name in zip(m.get_rhs_input(), before, ("u", "v", "η")):
+                assert_bitwise(x, y, name)
