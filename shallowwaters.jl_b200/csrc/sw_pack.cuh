@@ -62,7 +62,7 @@ struct Pack<float> {
         return r;
     }
     static __device__ __forceinline__ P mul(P a, P b, P nz) {
-#ifdef SWB_FAST_BUILD
+#if SWB_FAST_BUILD   // 0 or undefined in the parity build
         return mulx(a, b);
 #else
         P r;
