@@ -73,7 +73,9 @@ enum sw_error {
     SW_ERR_TIMEOUT = 4,      /* a bounded device wait ran out                    */
     SW_ERR_UNSUPPORTED = 5,  /* option combination not built                     */
     SW_ERR_NOMEM = 6,        /* device allocation failed                         */
-    SW_ERR_DEPARTURE = 7,    /* tracer departure point left the wrapped domain   */
+    SW_ERR_DEPARTURE = 7,    /* tracer departure point left the wrapped domain;  */
+                             /* u, v, eta are those of a whole step: that one,   */
+                             /* or up to 15 later where steps run in blocks      */
     SW_ERR_NODEVICE = 8      /* no CUDA device                                   */
 };
 

@@ -257,11 +257,12 @@ struct sw_ctx {
     // their events (see capture_block); null otherwise
     cudaStream_t side = nullptr;
     std::vector<cudaEvent_t>* side_events = nullptr;
+    bool side_last = false;       // the step being captured is the block's last
     std::map<unsigned, StepGraph> graphs;
     int nsm = 148;
     int tail_ty = TAIL_TY;        // rows per warp strip of the streaming tail (see pick_strip_ty)
     int stage_ty = STAGE_TY;      // rows per warp strip of the streaming stage and SSP momentum kernels
-    DevStatus* dst = nullptr;     // device status
+    DevStatus* dst = nullptr;     // device status, and that of the tracers on a block's side branch
     DiagPartial* diag = nullptr;  // DIAG_BLOCKS partials + the result (allocated on first use)
     DevStatus* hst = nullptr;     // pinned host mirror
     int p = 0;                    // state parity
@@ -885,7 +886,9 @@ struct Engine : EngineBase {
         a.half_dtadvu = (T)c.half_dtadvu; a.half_dtadvv = (T)c.half_dtadvv;
         a.jSST = (T)c.jSST; a.SSTmin = (T)c.SSTmin;
         a.gr = rule(ctx);
-        a.st = ctx->dst;
+        a.run = ctx->dst;
+        a.st = ctx->side ? ctx->dst + 1 : ctx->dst;
+        a.last = ctx->side && ctx->side_last;
         return a;
     }
 
@@ -1672,6 +1675,7 @@ int capture_block(sw_ctx* ctx, long long i, int n, sw_ctx::StepGraph& sg) {
         ctx->side_events = &events;
         for (int k = 0; k < n && !rc && e == cudaSuccess; k++) {
             if (branch && k >= 2) e = cudaStreamWaitEvent(ctx->stream, events[2 * (k - 2) + 1]);
+            ctx->side_last = k == n - 1;
             if (e == cudaSuccess) rc = ctx->eng->step(ctx, i + k);
             ctx->p = 1 - ctx->p;
         }
@@ -1865,7 +1869,7 @@ int state_copy_in(sw_ctx* ctx, const void* u, const void* v, const void* eta, co
     if ((rc = copy_in(ctx, ctx->S[0].v, v, shape_v(ctx->g)))) return rc;
     if ((rc = copy_in(ctx, ctx->S[0].e, eta, shape_e(ctx->g)))) return rc;
     if ((rc = copy_in(ctx, ctx->sst[0], sst, shape_s(ctx->g)))) return rc;
-    CK(cudaMemsetAsync(ctx->dst, 0, sizeof(DevStatus), ctx->stream));
+    CK(cudaMemsetAsync(ctx->dst, 0, 2 * sizeof(DevStatus), ctx->stream));
     CK(cudaMemsetAsync(ctx->sched, 0, sizeof(TileSched), ctx->stream));
     return SW_OK;
 }
@@ -2671,7 +2675,7 @@ int sw_create(const sw_config* cfg, const sw_static* st, sw_ctx** out) {
     }
     {
         void* p = nullptr;
-        if ((rc = alloc(&p, sizeof(DevStatus)))) return rc;
+        if ((rc = alloc(&p, 2 * sizeof(DevStatus)))) return rc;
         ctx->dst = static_cast<DevStatus*>(p);
         if ((rc = alloc(&p, sizeof(TileSched)))) return rc;
         ctx->sched = static_cast<TileSched*>(p);

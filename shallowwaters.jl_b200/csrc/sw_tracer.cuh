@@ -27,7 +27,13 @@ struct TracerArgs {
     T dtadvu, dtadvv, half_dtadvu, half_dtadvv;
     T jSST, SSTmin;
     GhostRule<Tp> gr;
+    // Where a bad departure point is reported, and the run's status.  They are
+    // the same, but for a tracer that runs beside the next step: a stop seen by
+    // some blocks of that step alone would leave its state torn.  The last
+    // tracer of such a branch, which no step runs beside, passes the report on.
     DevStatus* st;
+    DevStatus* run;
+    bool last;
 };
 
 // Julia's Int(floor(x)); NaN, Inf and indices no array can take are flagged.
@@ -80,13 +86,21 @@ struct TracerIONative {
     __device__ __forceinline__ ES operator()(Tp x) const { return x; }   // Tprog value -> sst element
 };
 
+__device__ __forceinline__ void report_departure(DevStatus* st) {
+    atomicCAS(&st->error, 0, (int)SW_ERR_DEPARTURE);
+    atomicExch(&st->stop, 1);
+}
+
 // 2-D launch: x over columns, y over rows (grid-stride in y)
 // The tracer for column block bx and rows by, by + gy, ... (128 threads).
 template <class T, class Tp, bool PER, bool UM_IS_U, bool CONS, class IO = TracerIONative<T, Tp>>
 __device__ __forceinline__ void tracer_body(const TracerArgs<T, Tp>& A, int bx, int by, int gy, const IO& io = IO()) {
     using EU = typename IO::EU;
     using ES = typename IO::ES;
-    if (A.st->stop) return;
+    if (A.st->stop || A.run->stop) {
+        if (A.last && A.st->stop && bx == 0 && by == 0 && threadIdx.x == 0) report_departure(A.run);
+        return;
+    }
     const Geom& g = A.g;
     const int N = g.N, M = g.M;
     const int a = bx * 128 + threadIdx.x;
@@ -165,8 +179,8 @@ __device__ __forceinline__ void tracer_body(const TracerArgs<T, Tp>& A, int bx, 
         if (gx) A.gr.sst(psst_o, g, a, b, out, io);             // ghost_points_sst! (:40)
     }
     if (bad) {   // the reference throws here; halt the device-side loop
-        atomicCAS(&A.st->error, 0, (int)SW_ERR_DEPARTURE);
-        atomicExch(&A.st->stop, 1);
+        report_departure(A.st);
+        if (A.last) report_departure(A.run);
     }
 }
 
