@@ -111,8 +111,24 @@ BlockCache& block_cache() {
 }
 constexpr size_t CACHE_LIMIT = size_t(16) << 30;
 
+// Returns the kept device blocks of the current device and CUDA context to
+// CUDA.  Those of others stay: freeing them would change the caller's context.
+void release_blocks_here() {
+    int d = 0;
+    cudaGetDevice(&d);
+    const unsigned long long cid = current_context_id();
+    BlockCache& c = block_cache();
+    std::lock_guard<std::mutex> lock(c.mu);
+    for (auto it = c.dev.begin(); it != c.dev.end();) {
+        if (it->first.device != d || it->first.context != cid) { ++it; continue; }
+        cudaFree(it->second);
+        c.cached -= it->first.bytes;
+        it = c.dev.erase(it);
+    }
+}
 // returns every kept device block to CUDA
 void release_cached_blocks() {
+    release_blocks_here();
     BlockCache& c = block_cache();
     std::lock_guard<std::mutex> lock(c.mu);
     int cur = 0;
@@ -122,7 +138,7 @@ void release_cached_blocks() {
         if (cudaSetDevice(kv.first.device) != cudaSuccess) continue;
         if (current_context_id() == kv.first.context) cudaFree(kv.second);
     }
-    cudaSetDevice(cur);
+    if (!c.dev.empty()) cudaSetDevice(cur);
     c.dev.clear();
     c.cached = 0;
 }
@@ -144,7 +160,7 @@ cudaError_t cached_malloc(void** p, size_t bytes) {
     const cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation) return e;
     (void)cudaGetLastError();
-    release_cached_blocks();          // a block that does not fit beside the kept ones
+    release_blocks_here();            // a block that does not fit beside the kept ones
     return cudaMalloc(p, bytes);
 }
 void cached_free(void* p, size_t bytes) {
