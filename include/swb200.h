@@ -239,12 +239,12 @@ int sw_run_timed(sw_ctx* ctx, int64_t nsteps, int64_t l2_flush_bytes,
                  double* step_ms_total, sw_status* status);
 /* Number of CUDA kernel launches the library has issued on this context. */
 int64_t sw_kernel_launches(const sw_ctx* ctx);
-/* Ends a context.  Its device blocks, and those of sw_adjoint_run, are kept by
- * the library for reuse by later calls of the same sizes (up to 16 GiB in all,
- * given back where a later allocation does not fit), so repeated calls do not
- * pay for cudaMalloc/cudaFree; sw_trim_memory frees them.  No reference
- * counterpart (the reference's preallocate! arrays are freed by Julia's
- * garbage collector). */
+/* Ends a context.  Its device blocks are kept by the library for reuse by later
+ * contexts of the same sizes (up to 16 GiB per CUDA context, and 4 GiB of those
+ * of sw_adjoint_run; the oldest go first, and all where a later allocation does
+ * not fit), so repeated calls do not pay for cudaMalloc/cudaFree;
+ * sw_trim_memory frees them.  No reference counterpart (the reference's
+ * preallocate! arrays are freed by Julia's garbage collector). */
 void sw_destroy(sw_ctx* ctx);
 /* Returns every device and pinned block kept for reuse to CUDA.  Call it with
  * no context in use. */

@@ -1,5 +1,6 @@
-// sw_pool.h -- device blocks kept by the library for reuse (sw_runtime.cu):
-// bounded, keyed by size, device and CUDA context, returned by sw_trim_memory.
+// sw_pool.h -- device blocks of the gradient, kept for reuse (sw_runtime.cu) in
+// a pool of their own: bounded, keyed by size, device and CUDA context, the
+// oldest going first, returned by sw_trim_memory.
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>

@@ -84,125 +84,157 @@ struct Fields3 { void* u = nullptr; void* v = nullptr; void* e = nullptr; };
 // Device and pinned blocks released by sw_destroy are kept for reuse by later
 // contexts of the same sizes: a drop-in call (create, run, destroy) then costs
 // no cudaMalloc/cudaFree after the first, which are slow and, for cudaFree,
-// erratic (milliseconds to a second).  At most CACHE_LIMIT bytes of device
-// memory are held; sw_trim_memory returns them all.  Device blocks are keyed
-// by the CUDA context that allocated them (current_context_id), so a block of
-// a context that was destroyed meanwhile is never handed out again.
+// erratic (milliseconds to a second).  Blocks are kept per device and CUDA
+// context (current_context_id), so a block of a context that was destroyed
+// meanwhile is never handed out again.  A pool holds at most `limit` bytes for
+// each; beyond it the blocks kept longest go back to CUDA, so sizes that are
+// not asked for again do not shut out the ones in use.  sw_trim_memory returns
+// them all.
 namespace {
-struct DevKey {
-    int device;
-    unsigned long long context;
-    size_t bytes;
-    bool operator<(const DevKey& o) const {
-        if (device != o.device) return device < o.device;
-        if (context != o.context) return context < o.context;
-        return bytes < o.bytes;
+class BlockPool {
+public:
+    explicit BlockPool(size_t limit_) : limit(limit_) {}
+    // a kept block of this size, or null
+    void* take(size_t bytes) {
+        Kept* k;
+        std::lock_guard<std::mutex> lock(mu);
+        if (!(k = here(false))) return nullptr;
+        auto it = k->blocks.find(bytes);
+        if (it == k->blocks.end()) return nullptr;
+        void* const p = it->second.first;
+        k->age.erase(it->second.second);
+        k->blocks.erase(it);
+        k->held -= bytes;
+        return p;
     }
-};
-struct BlockCache {
+    void give(void* p, size_t bytes) {
+        std::vector<void*> out;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            Kept* k = bytes <= limit ? here(true) : nullptr;
+            if (!k) {
+                out.push_back(p);
+            } else {
+                auto it = k->blocks.insert({bytes, {p, ++clock}});
+                k->age[clock] = it;
+                k->held += bytes;
+                while (k->held > limit) {
+                    it = k->age.begin()->second;
+                    out.push_back(it->second.first);
+                    k->held -= it->first;
+                    k->blocks.erase(it);
+                    k->age.erase(k->age.begin());
+                }
+            }
+        }
+        for (void* q : out) cudaFree(q);
+    }
+    // returns the blocks of the current device and CUDA context
+    void release_here() {
+        std::lock_guard<std::mutex> lock(mu);
+        Kept* k = here(false);
+        if (!k) return;
+        for (auto& b : k->blocks) cudaFree(b.second.first);
+        *k = Kept();
+    }
+    // returns every block; those of a context that no longer exists are dropped, not freed
+    void release_all() {
+        release_here();
+        std::lock_guard<std::mutex> lock(mu);
+        int cur = 0;
+        cudaGetDevice(&cur);
+        for (auto& d : kept) {
+            if (d.second.blocks.empty() || cudaSetDevice(d.first.first) != cudaSuccess) continue;
+            if (current_context_id() != d.first.second) continue;
+            for (auto& b : d.second.blocks) cudaFree(b.second.first);
+        }
+        cudaSetDevice(cur);
+        kept.clear();
+    }
+
+private:
+    struct Kept {
+        using Blocks = std::multimap<size_t, std::pair<void*, unsigned long long>>;   // by size: address, time kept
+        Blocks blocks;
+        std::map<unsigned long long, Blocks::iterator> age;                           // oldest first
+        size_t held = 0;
+    };
+    Kept* here(bool make) {
+        int d = 0;
+        cudaGetDevice(&d);
+        const unsigned long long cid = current_context_id();
+        if (!cid) return nullptr;
+        auto it = kept.find({d, cid});
+        if (it == kept.end()) {
+            if (!make) return nullptr;
+            it = kept.emplace(std::make_pair(d, cid), Kept()).first;
+        }
+        return &it->second;
+    }
+    const size_t limit;
     std::mutex mu;
-    std::multimap<DevKey, void*> dev;
-    std::multimap<size_t, void*> pinned;
-    size_t cached = 0;
+    std::map<std::pair<int, unsigned long long>, Kept> kept;
+    unsigned long long clock = 0;
 };
-BlockCache& block_cache() {
-    static BlockCache* c = new BlockCache();   // never destroyed: may be used during process exit
+// The pools are never destroyed: they may be used during process exit.
+BlockPool& context_blocks() {
+    static BlockPool* p = new BlockPool(size_t(16) << 30);
+    return *p;
+}
+// The gradient's blocks have a pool of their own: its records are gigabytes of
+// a size that is new for every grid and number of steps (512x256 Float64 over
+// 60 steps: 2.7 GB in all).
+BlockPool& gradient_blocks() {
+    static BlockPool* p = new BlockPool(size_t(4) << 30);
+    return *p;
+}
+struct PinnedCache {
+    std::mutex mu;
+    std::multimap<size_t, void*> blocks;
+};
+PinnedCache& pinned_cache() {
+    static PinnedCache* c = new PinnedCache();
     return *c;
 }
-constexpr size_t CACHE_LIMIT = size_t(16) << 30;
 
-// Returns the kept device blocks of the current device and CUDA context to
-// CUDA.  Those of others stay: freeing them would change the caller's context.
-void release_blocks_here() {
-    int d = 0;
-    cudaGetDevice(&d);
-    const unsigned long long cid = current_context_id();
-    BlockCache& c = block_cache();
-    std::lock_guard<std::mutex> lock(c.mu);
-    for (auto it = c.dev.begin(); it != c.dev.end();) {
-        if (it->first.device != d || it->first.context != cid) { ++it; continue; }
-        cudaFree(it->second);
-        c.cached -= it->first.bytes;
-        it = c.dev.erase(it);
-    }
-}
-// returns every kept device block to CUDA
-void release_cached_blocks() {
-    release_blocks_here();
-    BlockCache& c = block_cache();
-    std::lock_guard<std::mutex> lock(c.mu);
-    int cur = 0;
-    cudaGetDevice(&cur);
-    for (auto& kv : c.dev) {
-        // blocks of a context that no longer exists are dropped, not freed
-        if (cudaSetDevice(kv.first.device) != cudaSuccess) continue;
-        if (current_context_id() == kv.first.context) cudaFree(kv.second);
-    }
-    if (!c.dev.empty()) cudaSetDevice(cur);
-    c.dev.clear();
-    c.cached = 0;
-}
-cudaError_t cached_malloc(void** p, size_t bytes) {
-    int d = 0;
-    cudaGetDevice(&d);
-    const unsigned long long cid = current_context_id();
-    if (cid) {
-        BlockCache& c = block_cache();
-        std::lock_guard<std::mutex> lock(c.mu);
-        auto it = c.dev.find({d, cid, bytes});
-        if (it != c.dev.end()) {
-            *p = it->second;
-            c.dev.erase(it);
-            c.cached -= bytes;
-            return cudaSuccess;
-        }
-    }
+cudaError_t pooled_malloc(BlockPool& pool, void** p, size_t bytes) {
+    if ((*p = pool.take(bytes))) return cudaSuccess;
     const cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation) return e;
     (void)cudaGetLastError();
-    release_blocks_here();            // a block that does not fit beside the kept ones
+    // a block that does not fit beside the kept ones; those of other devices
+    // and CUDA contexts stay, as freeing them would change the caller's
+    context_blocks().release_here();
+    gradient_blocks().release_here();
     return cudaMalloc(p, bytes);
 }
-void cached_free(void* p, size_t bytes) {
-    int d = 0;
-    cudaGetDevice(&d);
-    const unsigned long long cid = current_context_id();
-    if (cid) {
-        BlockCache& c = block_cache();
-        std::lock_guard<std::mutex> lock(c.mu);
-        if (c.cached + bytes <= CACHE_LIMIT) {
-            c.dev.insert({{d, cid, bytes}, p});
-            c.cached += bytes;
-            return;
-        }
-    }
-    cudaFree(p);
-}
+cudaError_t cached_malloc(void** p, size_t bytes) { return pooled_malloc(context_blocks(), p, bytes); }
+void cached_free(void* p, size_t bytes) { context_blocks().give(p, bytes); }
 cudaError_t cached_malloc_host(void** p, size_t bytes) {
     {
-        BlockCache& c = block_cache();
+        PinnedCache& c = pinned_cache();
         std::lock_guard<std::mutex> lock(c.mu);
-        auto it = c.pinned.find(bytes);
-        if (it != c.pinned.end()) {
+        auto it = c.blocks.find(bytes);
+        if (it != c.blocks.end()) {
             *p = it->second;
-            c.pinned.erase(it);
+            c.blocks.erase(it);
             return cudaSuccess;
         }
     }
     return cudaMallocHost(p, bytes);
 }
 void cached_free_host(void* p, size_t bytes) {
-    BlockCache& c = block_cache();
+    PinnedCache& c = pinned_cache();
     std::lock_guard<std::mutex> lock(c.mu);
-    c.pinned.insert({bytes, p});
+    c.blocks.insert({bytes, p});
 }
 }  // namespace
 
 namespace swb {
-// The adjoint's blocks come from the same cache: at 512x256 Float64 over 60
-// steps their cudaMalloc and cudaFree were 14 of a gradient's 34 ms.
-cudaError_t pool_malloc(void** p, size_t bytes) { return cached_malloc(p, bytes); }
-void pool_free(void* p, size_t bytes) { cached_free(p, bytes); }
+// The adjoint's blocks are kept too: at 512x256 Float64 over 60 steps their
+// cudaMalloc and cudaFree were 14 of a gradient's 34 ms.
+cudaError_t pool_malloc(void** p, size_t bytes) { return pooled_malloc(gradient_blocks(), p, bytes); }
+void pool_free(void* p, size_t bytes) { gradient_blocks().give(p, bytes); }
 }  // namespace swb
 
 struct sw_ctx;
@@ -2617,11 +2649,12 @@ void sw_batch_destroy(sw_batch* b) {
 
 int sw_trim_memory(void) {
     release_dropin_contexts();
-    release_cached_blocks();
-    BlockCache& c = block_cache();
+    context_blocks().release_all();
+    gradient_blocks().release_all();
+    PinnedCache& c = pinned_cache();
     std::lock_guard<std::mutex> lock(c.mu);
-    for (auto& kv : c.pinned) cudaFreeHost(kv.second);
-    c.pinned.clear();
+    for (auto& kv : c.blocks) cudaFreeHost(kv.second);
+    c.blocks.clear();
     return SW_OK;
 }
 

@@ -45,6 +45,40 @@ assert room() >= before + GIB, "the context's own blocks were given back"
 print("done")
 """
 
+NEWEST = """
+import numpy as np
+from swb200 import Model, Parameter, model_setup
+S = model_setup(Parameter(nx=1000, Ndays=1.0))
+Model(S).close()                       # makes the primary context
+lib.sw_trim_memory()
+start = room()
+sizes = [GIB + k * (64 << 20) for k in range(14)]
+for n in sizes:                        # 19.7 GiB of blocks that nothing asks for again
+    p, e = take(n)
+    assert e == 0
+    free(p, n)
+assert start - room() <= 4 * GIB + (64 << 20), "the gradient's pool"
+p, e = take(sizes[-1])
+before = room()
+free(p, sizes[-1])
+assert e == 0 and room() == before, "the newest is kept"
+model = lambda: Model(S).close()
+before = room()
+model()
+assert room() < before, "a model's blocks are kept beside them"
+before = room()
+model()
+assert room() == before
+big, e = take(5 * GIB)
+assert e == 0
+before = room()
+free(big, 5 * GIB)
+assert room() >= before + 5 * GIB, "a block above the limit goes back at once"
+lib.sw_trim_memory()
+assert room() >= start - (64 << 20)
+print("done")
+"""
+
 
 def child(code):
     r = subprocess.run([sys.executable, "-c", POOL + code], capture_output=True, text=True, timeout=300,
@@ -56,3 +90,9 @@ def test_an_allocation_that_does_not_fit_leaves_the_context():
     """It gives back what is kept for the caller's CUDA context, and the
     caller's context stays the current one."""
     child(OUT_OF_MEMORY)
+
+
+def test_the_newest_blocks_are_kept():
+    """The gradient's blocks stay within their bound, the oldest go first, and
+    they do not keep a model's blocks out."""
+    child(NEWEST)
