@@ -60,10 +60,15 @@ bool member_tiles(const ShapeInfo& f, const Geom& g, int h, int& ntx, int& nty, 
 
 int step_batch_plan(const Geom* gs, int n, int nsm, StepPlan* plans) {
     const auto info = shape_infos<float, true>();
+    // force a shape and the most rows per tile, as for a lone context (plan_of)
+    const char* env = getenv("SWB200_STEP");
+    const char* envr = getenv("SWB200_STEP_ROWS");
+    const int only = env ? atoi(env) : NSHAPES, rows = envr ? atoi(envr) : 0;
     int best = -1, best_h = 0;
     double cost = 1e30;
-    for (int s = 0; s < NSHAPES; s++)
-        for (int h = info[s].EH; h >= 2; h -= h > 16 ? 4 : 2) {
+    for (int s = 0; s < NSHAPES; s++) {
+        if (only < NSHAPES && s != only) continue;
+        for (int h = rows > 0 ? std::max(rows, 2) : info[s].EH; h >= 2; h -= rows > 0 ? h : h > 16 ? 4 : 2) {
             double total = 0, longest = 0;
             bool ok = true;
             for (int m = 0; m < n && ok; m++) {
@@ -77,6 +82,7 @@ int step_batch_plan(const Geom* gs, int n, int nsm, StepPlan* plans) {
             const double c = total / nsm + 0.5 * longest;
             if (ok && c < cost) { cost = c; best = s; best_h = h; }
         }
+    }
     for (int m = 0; m < n && best >= 0; m++) {
         double c;
         plans[m].shape = best;
