@@ -547,8 +547,9 @@ def main():
             "e2e": e2e,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": ncu_traffic(cells) if storage == "native" and not main["whole"] else None,
-                         "kernel": "rk_step_kernel" if main["whole"] else
-                         "rk_stage_tma" if storage == "native" else "s16_stage_kernel",
+                         "kernel": {(True, True): "rk_step_kernel", (True, False): "s16_step_kernel",
+                                    (False, True): "rk_stage_tma", (False, False): "s16_stage_kernel"}[
+                                        bool(main["whole"]), storage == "native"],
                          "bytes_per_cell": stage_bytes,
                          "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
                          else "fallback 6.65 TB/s"},

@@ -16,8 +16,8 @@
 // the tail reads +-2, so RKo = 4 needs 10 points below and 6 above a tile;
 // halo points are computed redundantly, on rows whose number shrinks from
 // stage to stage.  Walls need no extra halo: ghost points are filled in shared
-// memory after each stage, by the rules of sw_ghost.cuh.  Where a periodic tile crosses x = 0 it holds the ghost
-// columns of both sides: its columns run
+// memory after each stage, by the rules of sw_ghost.cuh.  Where a periodic tile
+// crosses x = 0 it holds the ghost columns of both sides: its columns run
 //   ..., N-2, N-1, N, N+1 | -2, -1, 0, 1, ...
 // so every column sees the neighbours and the depth that the reference's
 // arrays give it, and a ghost column is 4 columns from its source.  A domain
@@ -31,21 +31,25 @@
 //
 // Order at the start.  What no earlier launch writes (a thread's columns and
 // ghost places, the rows' static fields) is formed before the wait for the
-// launch before, which it overlaps: 64x32 12.6 -> 10.8 us a step, 512x256
-// 23.8 -> 22.4.  The stop flag is read beside the state.
+// launch before, which it overlaps: without that 64x32 takes 1.8 us a step more,
+// 512x256 1.4.  The stop flag is read beside the state.
 //
-// Measured (B200, us per step with the tracer beside it; the four stage
-// launches and the tail before): 64x32 22.6 -> 10.0, 256x128 25.6 -> 10.8,
-// 512x256 48.7 -> 19.6, 1000x500 over a ridge 88 -> 37.8, 2048x1024 181 -> 123,
-// 512x256 Float64 60 -> 23.1, SSPRK3 500x250 41.8 -> 26.0.  The 103 x 47 tile
-// of 63 rows takes 65 thousand clocks: load 6, A 4 x 4.2, B 4 x 7.5, T1 and
-// T2 11, the rest start and end.  A third of the issue slots are used (sixteen
-// warps of 128 registers); a warp waits most for the fixed latency of its
-// packed adds, then for barriers, loads and the shared memory about equally.
-// 20, 24 and 32 warps with fewer registers, passes A, T1 and T2 unrolled by 4
-// and a division on packs took as long or longer.  A tile of a small grid
-// takes 13 thousand clocks, 700 to 1100 a pass, which are the latencies of one
-// row, and the launch.
+// Measured (B200, us per step in blocks of steps, Smagorinsky and quadratic
+// drag, the tracer of every step beside the next; the launches per stage, then
+// this kernel):
+//                     64x32       512x256     2048x1024   2999x1499
+//   Float32        25.4    9.4  52.3  20.0    202  137    376  291
+//   Float64        27.6    8.6  60.9  24.0    514  243    880  521
+//   SSPRK3         35.1   13.8  46.3  25.8    338  155    641  350
+//   bf16 storage   70.0   11.2  76.0  23.3    308  169    584  359
+// What bounds it: the latency of its passes.  At 2048x1024 it takes 124 us alone
+// for three waves of tiles; 45 % of the issue slots are used, the shared-memory
+// pipe 49 %, the FMA pipe 34 %, DRAM 3 %, and a warp waits, per issue, 1.8
+// cycles for the fixed latency of its packed adds, 1.2 for global loads, 0.8 each
+// for barriers and shared memory (sixteen warps of 128 registers, all that the
+// register file holds).  20, 24 and 32 warps with fewer registers, passes A, T1
+// and T2 unrolled by 4 and a division on packs took as long or longer.  On a
+// small grid a pass is one row's latency, and a step little but its ten passes.
 #pragma once
 #include <type_traits>
 
@@ -181,10 +185,12 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, const IO& io, ty
     const P half = A.half, q4 = A.q4, nz = A.nz;
     const bool lowwall = zy == -2, highwall = zy1 == M + 2;
 
-    // This warp's rows of [from, to) in the passes that keep nothing in registers from one to the next: an equal share,
-    // as the rows shrink from stage to stage and a tile's outputs are half to three quarters of its rows (512x256 21.5
-    // -> 19.6 us a step, 2048x1024 125 -> 122.7, SSPRK3 200x100 Float64 26.7 -> 19.8).  With one row per thread its own,
-    // which is known not to loop (64x32 10.1 against 11.3).
+    // This warp's rows of [from, to) in the passes that keep nothing in
+    // registers from one to the next: an equal share, as the rows shrink from
+    // stage to stage and a tile's outputs are half to three quarters of its rows
+    // (its own rows instead take longer: 512x256 1.9 us a step, 2048x1024 2.3,
+    // SSPRK3 200x100 Float64 6.9).  With one row per thread its own, which is
+    // known not to loop (64x32 1.2 us less).
     auto share = [&](int from, int to, int& r0, int& r1) {
         if constexpr (R == 1) {
             r0 = max(ly0, from);
@@ -335,9 +341,11 @@ __device__ __forceinline__ void step_tile(const StepArgs<T>& A, const IO& io, ty
         }
         return G;
     };
-    // What the stages need of them, in one register each (found anew in each stage they took 500 of a ghost pass's
-    // 900 clocks, kept as they are the registers of the four-row tiles and more): source, place and its mark, and what eta does (1 the same,
-    // 2 and 3 the row after or before: the corners) or which of u and eta there is.
+    // What the stages need of them, in one register each (found anew in each
+    // stage they took 500 of a ghost pass's 900 clocks, kept as they are the
+    // registers of the four-row tiles and more): source, place and its mark, and
+    // what eta does (1 the same, 2 and 3 the row after or before: the corners) or
+    // which of u and eta there is.
     static_assert(NP * V <= 8192, "13 bits for a place");
     int col_ghost = -1, row_ghost = -1;
     if (EDGE) {

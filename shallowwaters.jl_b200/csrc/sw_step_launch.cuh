@@ -13,13 +13,17 @@ namespace {
 
 // Tile shapes (StepShape: warps side by side, warps, rows per thread).  Low
 // tiles for grids that leave SMs idle: a pass is then one row's latency, and
-// more rows per block cost more clocks than their halos (64x32: 20 rows 10.0 us
-// a step, 24 10.5, 32 11.6; 256x128 needs 24 rows to run in one wave, 10.8
-// against 18.6).  32 rows fill the gap up to 512x256 (400x200: 13.5, else
-// 15.7), 2 warps side by side the ones above (512x256: 19.6 against 22.2).
+// more rows per block cost more clocks than their halos (Float32, us a step,
+// 64x32: 20 rows 9.5, 24 10.0, 32 11.0; 256x128 needs 24 rows to run in one
+// wave, 10.8 against 18.7).  32 rows fill the gap up to 512x256 (400x200: 13.5,
+// else 15.7), 2 warps side by side the ones above (512x256: 20.0 against 22.5).
 // The last shape fills the shared memory of an SM, for several waves
-// (2048x1024: 123 against 164); with a depth that varies along x the eighth
+// (2048x1024: 137 against 170); with a depth that varies along x the eighth
 // array costs it rows.
+// 24 warps leave 80 registers a thread, which spills 16 to 84 bytes (164 in a
+// batch); where that shape is picked the next one, which spills nothing, is
+// slower all the same (256x128: 11.8 against 10.8, SSPRK3 128x64 15.5 against
+// 13.8).
 template <class T, bool HVAR>
 struct Shapes;
 template <bool HVAR>
@@ -59,7 +63,11 @@ std::array<ShapeInfo, NSHAPES> shape_infos() {
     };
     return {of(typename SS::S0{}), of(typename SS::S1{}), of(typename SS::S2{}), of(typename SS::S3{}), of(typename SS::S4{})};
 }
-// a tile's clocks: its passes' latencies and barriers, and its rows, measured
+// a tile's clocks: its passes' latencies and barriers, and its rows, measured.
+// One line serves all forms, as only the order of the shapes matters: of the
+// five forced in turn it picks the fastest (within 1 %) for Float32, Float64,
+// SSPRK3, SSPRK2 with Sadourny in Float64 and bf16 storage at each of seven
+// sizes from 64x32 to 2999x1499.
 inline double tile_clocks(const ShapeInfo& f, int rows) { return 7000.0 + 540.0 * f.EWW * rows; }
 
 template <class T, bool HVAR>

@@ -2,8 +2,11 @@
 // tiles of sw_step.cuh with Float32 arithmetic, the state read and written as
 // pairs (Step16).  The stage increments, which the launches per stage keep in
 // memory as 16-bit arrays, are rounded to that form and stay in the tile.
-// us per step against the launches per stage (B200): 2048x1024 bf16 287 -> 181,
-// 1000x500 f16 78 -> 58, 200x100 bf16 69 -> 16.
+// us per step with the tracer beside it (B200, bf16; the launches per stage,
+// then this): 64x32 70 and 11.2, 512x256 76 and 23.3, 1024x512 95 and 50.9,
+// 2048x1024 308 and 169.  Its tallest tiles spill (8 rows 120 bytes in bf16 and
+// 84 in half, 7 rows 80) and are the faster ones all the same: 2048x1024 takes
+// 198 us in the next shape, which spills nothing.
 #include "sw_step_launch.cuh"
 
 namespace swb {
