@@ -206,6 +206,8 @@ int sw_get_state(sw_ctx* ctx, void* u, void* v, void* eta, void* sst);
  * the values of that evaluation (src/PV_advection.jl:2-18, src/rhs.jl:89-128);
  * they follow from this state, H and f_q.  Where a step is one launch that
  * input is formed again from the step's start when this call asks for it.
+ * After SW_ERR_DEPARTURE it is the input of one of the steps since the last
+ * NaN check, not of a particular one.
  * Native storage only. */
 int sw_get_rhs_input(sw_ctx* ctx, void* u, void* v, void* eta);
 /* FP64 reductions over the current state. */
